@@ -567,7 +567,7 @@ struct AdjTraceHook {
     }
     __device__ void photon_begin(const Lane &) { nv = 0; overflow = 0; direct_hit = 0; seg_entries = 0; }
     __device__ void march_begin() { ++seg_entries; }
-    __device__ void accepted() { ++seg_entries; }
+    __device__ void accepted(int n) { seg_entries += n; }
     // each hook ends a segment: the direct march at EV_SCATTER, a move at EV_VERTEX, a connection
     // at EV_SCATTER_ONCE
     __device__ bool at(Lane &L, int ev) {
@@ -983,14 +983,16 @@ adjoint_trace_event_kernel(const __grid_constant__ KParams P, const __grid_const
     if (h.nabort) atomicAdd(A.cnt + ADJ_ABORTED, h.nabort);
 }
 
-// the trace's tail: the live slots, with their checkpoints and hook state, on the persistent lane loop
+// the trace's tail: the live slots, with their checkpoints and hook state, on the persistent lane loop,
+// spread over the warps as in wf_finish_kernel
 template <int FK>
-__global__ void __launch_bounds__(128, 4)
+__global__ void __launch_bounds__(128, lane_blocks(FK))
 adjoint_trace_finish_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveParams W,
                             const __grid_constant__ AdjParams A, int it) {
     const int lane = threadIdx.x & 31, cur = it & 1;
     const unsigned n0 = list_cnt(W, cur)[0], n = n0 + list_cnt(W, cur)[1];
-    const unsigned gid = blockIdx.x * blockDim.x + threadIdx.x, lanes = gridDim.x * blockDim.x;
+    const unsigned lanes = gridDim.x * blockDim.x;
+    const unsigned gid = (unsigned(lane) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * gridDim.x + blockIdx.x;
     if (gid == 0 && n > lanes) atomicAdd(P.counters + CNT_LOST, (unsigned long long)(n - lanes));
     Lane L;
     L.end = 0;
@@ -1098,7 +1100,7 @@ __global__ void __launch_bounds__(128, 3) adjoint_replay_kernel(const __grid_con
                 } else {                                // the connection from vertex k
                     restore(L, P, V[k], true);
                     L.mp = L.pos;
-                    Field<FK>::eval(F, L.tab, L.mp, L.s, L.mn, L.mg);
+                    field_at<FK>(F, L.tab, L.mp, L.s, L.mn, L.mg);
                     ev = EV_VERTEX;
                     h.stop_ev = EV_SCATTER_ONCE;
                 }
@@ -1149,11 +1151,13 @@ __global__ void __launch_bounds__(128, 3) adjoint_replay_kernel(const __grid_con
         if (live == 0) break;
         const int thr = max(1, (__popc(live) * A.idle_replay + 16) >> 5);
         if (__any_sync(kFull, mode == M_MARCH)) {
+            typename Field<FK>::Cache C;
+            C.clear();
             for (;;) {
                 if (mode == M_MARCH) {
                     for (int t = 0; t < 2; ++t) {
                         const float3 q = L.mp;
-                        const bool end = march_step<FK>(L, P);
+                        const bool end = march_step<FK>(L, P, C);
                         ++rsteps;
                         if (q.x != L.mp.x || q.y != L.mp.y || q.z != L.mp.z) {
                             if (base + h.seg_len < pend) A.traj[base + h.seg_len] = make_float4(L.mp.x, L.mp.y, L.mp.z, L.cur);

@@ -199,8 +199,21 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
+// The window bounds of a field within `dev` of `base` (dev < 0: unknown) whose gradient stays below
+// `grad` in the 1-norm; none unless n stays above half the base.
+static void set_field_bounds(FieldParams &F, double base, double dev, double grad) {
+    F.grad_bound = 0.0f;
+    F.n_low = 0.0f;
+    const double low = base - 1.01 * dev - 1e-4;
+    if (!(dev >= 0.0) || !(grad < 1e9) || !(low > 0.5 * base)) return;
+    F.grad_bound = float(1.01 * grad);
+    F.n_low = float(0.999 * low);
+}
+
 // Spline coefficients as float offsets from their mean (see spline_field in dev_field.cuh).
-static float spline_offsets(const smp_field_desc &f, std::vector<float> &delta) {
+// Fills F's base value and window bounds: the weights are convex, so n stays within the largest offset
+// of the base, and a derivative along an axis is a convex sum of coefficient differences along it.
+static void spline_offsets(const smp_field_desc &f, std::vector<float> &delta, FieldParams &F) {
     size_t n = size_t(f.grid_n[0]) * f.grid_n[1] * f.grid_n[2];
     double mean = 0.0;
     for (size_t i = 0; i < n; ++i) mean += f.grid_coeff[i];
@@ -208,7 +221,24 @@ static float spline_offsets(const smp_field_desc &f, std::vector<float> &delta) 
     float base = float(f.grid_offset + mean);
     delta.resize(n);
     for (size_t i = 0; i < n; ++i) delta[i] = float(double(f.grid_coeff[i]) + f.grid_offset - double(base));
-    return base;
+    F.spline_base = base;
+    const int N0 = f.grid_n[0], N1 = f.grid_n[1], N2 = f.grid_n[2];
+    const size_t s1 = size_t(N0), s2 = s1 * N1;
+    float dev = 0.0f, d0 = 0.0f, d1 = 0.0f, d2 = 0.0f;
+    bool finite = true;
+    for (int z = 0; z < N2; ++z)
+        for (int y = 0; y < N1; ++y) {
+            const float *r = delta.data() + z * s2 + y * s1;
+            for (int x = 0; x < N0; ++x) {
+                dev = std::max(dev, std::fabs(r[x]));
+                finite = finite && std::isfinite(r[x]);
+                if (x) d0 = std::max(d0, std::fabs(r[x] - r[x - 1]));
+                if (y) d1 = std::max(d1, std::fabs(r[x] - r[x - long(s1)]));
+                if (z) d2 = std::max(d2, std::fabs(r[x] - r[x - long(s2)]));
+            }
+        }
+    set_field_bounds(F, double(base), finite ? double(dev) : -1.0,
+                     double(d0) * F.xres[0] + double(d1) * F.xres[1] + double(d2) * F.xres[2]);
 }
 
 // Bessel table for the march: intervals of width h = 1/16 in x = k r up to x_max (<= 128). For
@@ -331,17 +361,25 @@ static void fill_field_params(const smp_field_desc &f, int fk, FieldParams &F) {
     F.bh = float(kBesselH);
     F.binv_h = float(1.0 / kBesselH);
     F.kb = F.k_r * F.binv_h;
-    // |grad n|_1 bounds for the march's checked windows. Bessel: |dn/dr| <= A k |J_m'| <= A k and
-    // |dn/(r dphi)| = A k m |J_m(x)|/x <= A k (J_{m-1} + J_{m+1} = 2m J_m / x), so |grad n|_1 <= 2 A k;
-    // the factor 4 leaves room for the table's interpolation error. Plane waves: sum |a_i| |k_i|_1.
-    F.grad_bound = 0.0f;
-    if (fk <= FK_BESSEL2) F.grad_bound = 4.0f * std::fabs(F.amp) * F.k_r;
-    if (fk == FK_PLANEWAVE) {
-        float G = 0.0f;
-        for (int i = 0; i < F.n_waves; ++i)
-            G += std::fabs(F.wamp[i]) * (std::fabs(F.wk[i][0]) + std::fabs(F.wk[i][1]) + std::fabs(F.wk[i][2]));
-        F.grad_bound = 2.0f * G;
+    // Bounds for the march's untested windows (the spline's come with its coefficients). Bessel, with
+    // |s| <= 1 (the clamp is at max_scaling; a negative one could let s past 1, then no bounds):
+    // |n - n_o| <= |A|; |dn/dr| <= |A| k |J_m'| <= |A| k and |dn/(r dphi)| = |A| k m |J_m(x)|/x
+    // <= |A| k, so |grad n|_1 <= 2 |A| k, twice that for the table's interpolation error. Plane waves:
+    // sum |a_i| and sum |a_i| |k_i|_1.
+    double dev = -1.0, grad = 0.0;
+    if (fk <= FK_BESSELN && !(F.max_scaling < 0.0f)) {
+        dev = std::fabs(double(F.amp));
+        grad = 4.0 * dev * double(F.k_r);
     }
+    if (fk == FK_PLANEWAVE) {
+        dev = 0.0;
+        for (int i = 0; i < F.n_waves; ++i) {
+            const double a = std::fabs(double(F.wamp[i]));
+            dev += a;
+            grad += 2.0 * a * (std::fabs(double(F.wk[i][0])) + std::fabs(double(F.wk[i][1])) + std::fabs(double(F.wk[i][2])));
+        }
+    }
+    set_field_bounds(F, double(F.n_o), dev, grad);
 }
 
 // The box test of traceTillBlock, p - L > -eps and R - p > -eps in float, as thresholds:
@@ -392,6 +430,10 @@ static void set_box_thresholds(KParams &k) {
         k.box_lo[i] = float_above(double(k.L[i]) - eps);
         k.box_hi[i] = float_below(double(k.R[i]) + eps);
     }
+    float m = 0.0f;
+    for (int i = 0; i < 3; ++i) m = std::max(m, std::max(std::fabs(k.L[i]), std::fabs(k.R[i])));
+    k.win_hmin = 6e-6f * m;
+    k.win_round = 1.1920929e-7f * m;
 }
 
 // LargeDist of movePhotonTillSensor (scene.cpp:627): 1e4 m in the reference; by default capped
@@ -480,6 +522,9 @@ struct smp_plan {
     int march_block = 128;      // threads per march-kernel block (128 or 256)
     bool tuned = false;         // the schedule came from smp_plan_tune
     size_t wave_cap = 0;        // slots the pool allocation holds
+    long long direct_max = 40000;   // renders of at most this many photons are one launch of the tail
+                                    // kernel, with no pool (SMP_WF_DIRECT)
+    long long finish_max = 1LL << 30;
     int wave_batch = 16;        // march/event launch pairs between live-slot checks
     int wave_split = 1;         // march lists and event queues by march class (WaveParams.split)
     void *d_wave = nullptr;
@@ -572,7 +617,7 @@ static int plan_setup_field(smp_plan *p, const smp_field_desc &f) {
     }
     if (p->fk == FK_SPLINE) {
         std::vector<float> delta;
-        p->kp.field.spline_base = spline_offsets(f, delta);
+        spline_offsets(f, delta, p->kp.field);
         cudaFree(p->d_coeff);
         p->d_coeff = nullptr;
         SMP_CUDA(cudaMalloc(&p->d_coeff, delta.size() * sizeof(float)));
@@ -631,6 +676,7 @@ static int plan_setup_field(smp_plan *p, const smp_field_desc &f) {
         p->kp.field.btab = p->d_btab;
         p->kp.field.bnodes = int(tab.size());
         p->kp.field.bint = int(tab.size() / 2);
+        p->kp.field.bend = float(p->kp.field.bint);
         p->smem_bytes = tab.size() * sizeof(float4);
     }
     set_step_sizes(p->kp, f);
@@ -710,6 +756,8 @@ int smp_plan_create(const smp_scene_desc *scene, const smp_medium_desc *medium, 
     if (const char *c = std::getenv("SMP_WF_SLOTS")) p->wave_slots_per_lane = std::max(1, std::min(16, std::atoi(c)));
     if (const char *c = std::getenv("SMP_WF_BLOCK")) p->march_block = std::atoi(c) == 256 ? 256 : 128;
     if (const char *c = std::getenv("SMP_WF_BATCH")) p->wave_batch = std::max(1, std::min(256, std::atoi(c)));
+    if (const char *c = std::getenv("SMP_WF_DIRECT")) p->direct_max = std::atoll(c);
+    if (const char *c = std::getenv("SMP_WF_FINISH")) p->finish_max = std::atoll(c);
     if (const char *c = std::getenv("SMP_WF_SPLIT")) p->wave_split = std::atoi(c) != 0;
     p->scene = *scene;
     p->medium = *medium;
@@ -851,23 +899,33 @@ static float photon_weight(const smp_scene_desc &s, int64_t n) {
 // kind needs more.
 static int wave_bricks(smp_plan *p);
 
+// The tail kernel's grid.
+static int finish_setup(smp_plan *p) {
+    WaveFn ff = wf_finish_fn(p->fk);
+    if (!ff) return set_error(SMP_ERR_BAD_ARG, "bad field kind");
+    int sms = 0, pf = 0;
+    int rc = allow_dynamic_smem(reinterpret_cast<const void *>(ff), p->smem_bytes);
+    if (rc) return rc;
+    SMP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
+    SMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, ff, kBlock, p->smem_bytes));
+    p->grid_finish = sms * std::max(pf, 1);
+    return SMP_OK;
+}
+
 static int wave_setup(smp_plan *p) {
     const bool bricks = p->fk == FK_SPLINE && p->bricks;
-    WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, bricks), fe = wf_event_fn(p->fk),
-           ff = wf_finish_fn(p->fk);
-    if (!fm || !fe || !ff) return set_error(SMP_ERR_BAD_ARG, "bad field kind");
+    WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, bricks), fe = wf_event_fn(p->fk);
+    if (!fm || !fe) return set_error(SMP_ERR_BAD_ARG, "bad field kind");
     p->march_smem = bricks ? size_t(kBrickSmemBytes) : p->smem_bytes;
-    int sms = 0, pm = 0, pe = 0, pf = 0;
+    int sms = 0, pm = 0, pe = 0;
     int rc = allow_dynamic_smem(reinterpret_cast<const void *>(fm), p->march_smem);
-    if (!rc) rc = allow_dynamic_smem(reinterpret_cast<const void *>(ff), p->smem_bytes);
+    if (!rc) rc = finish_setup(p);
     if (rc) return rc;
     SMP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
     SMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pm, fm, p->march_block, p->march_smem));
     SMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pe, fe, kBlock, 0));
-    SMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, ff, kBlock, p->smem_bytes));
     p->grid_march = sms * std::max(pm, 1);
     p->grid_event = sms * std::max(pe, 1);
-    p->grid_finish = sms * std::max(pf, 1);
     const size_t n = size_t(p->grid_march) * size_t(p->march_block) * size_t(p->wave_slots_per_lane);
     p->wp.chunk = p->wave_chunk;
     if (p->d_wave && p->wave_cap >= n) {            // the allocation holds this many slots
@@ -957,6 +1015,18 @@ static unsigned long long live_of(unsigned long long word) {
 // wave_batch pairs until no slot is live. The live count after each batch is read back while the
 // next batch is already queued, so the device does not idle during the check.
 static int wave_run(smp_plan *p, const KParams &k, cudaStream_t s) {
+    if (!p->bricks && k.n_photons <= p->direct_max) {
+        int rc = finish_setup(p);
+        if (rc) return rc;
+        KParams kd = k;
+        kd.fetch_from = std::min<long long>(k.n_photons, (long long)p->grid_finish * kBlock);
+        WaveParams W;
+        std::memset(&W, 0, sizeof(W));
+        wf_finish_fn(p->fk)<<<p->grid_finish, kBlock, p->smem_bytes, s>>>(kd, W, -1);
+        SMP_CUDA(cudaGetLastError());
+        p->n_launched += 1;
+        return SMP_OK;
+    }
     int rc = wave_setup(p);
     if (rc) return rc;
     WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, p->wp.nb > 0), fe = wf_event_fn(p->fk),
@@ -965,7 +1035,7 @@ static int wave_run(smp_plan *p, const KParams &k, cudaStream_t s) {
     const int mb = p->march_block;
     if (W.nb > 0) SMP_CUDA(cudaMemsetAsync(W.bcnt[0], 0, 2 * size_t(W.nb) * sizeof(unsigned), s));
     // once the live slots fit in one persistent grid, the finisher runs them to the end
-    const unsigned finish_at = unsigned(p->grid_finish) * unsigned(kBlock);
+    const unsigned finish_at = unsigned(std::min<long long>((long long)p->grid_finish * kBlock, p->finish_max));
     SMP_CUDA(cudaMemsetAsync(W.cnt, 0, 8 * sizeof(unsigned), s));
     fe<<<p->grid_event, kBlock, 0, s>>>(k, W, -1);
     SMP_CUDA(cudaGetLastError());
@@ -1477,7 +1547,7 @@ int smp_field_eval(const smp_field_desc *field, double scaling, int64_t n_points
     }
     if (fk == FK_SPLINE && e == cudaSuccess) {
         std::vector<float> delta;
-        F.spline_base = spline_offsets(*field, delta);
+        spline_offsets(*field, delta, F);
         e = cudaMalloc(&d_coeff, delta.size() * sizeof(float));
         if (e == cudaSuccess) e = cudaMemcpy(d_coeff, delta.data(), delta.size() * sizeof(float), cudaMemcpyHostToDevice);
         F.coeff = d_coeff;
@@ -1491,6 +1561,7 @@ int smp_field_eval(const smp_field_desc *field, double scaling, int64_t n_points
         F.btab = d_tab;
         F.bnodes = int(tab.size());
         F.bint = int(tab.size() / 2);
+        F.bend = float(F.bint);
     }
     size_t np = size_t(n_points);
     if (e == cudaSuccess) e = cudaMalloc(&d_pts, np * 3 * sizeof(double));
@@ -1676,6 +1747,7 @@ static int batch_set(BatchRun &b, const smp_instance_desc *instances) {
         fill_field_params(d.field, fk, I.field);
         I.field.bnodes = 2 * b.tab_int[fk];
         I.field.bint = b.tab_int[fk];
+        I.field.bend = float(I.field.bint);
         I.field.btab = b.d_tabs + b.tab_off[fk];
         I.film = static_cast<char *>(b.d_films) + px * bpp * size_t(i);
         I.sigma_t = float(d.medium.sigma_t);                      // medium.h:24-38
@@ -2536,6 +2608,7 @@ extern "C" int smp_render_noalloc(const smp_scene_desc *scene, const smp_medium_
         k.field.btab = d_tab;
         k.field.bnodes = tab_entries;
         k.field.bint = tab_entries / 2;
+        k.field.bend = float(k.field.bint);
         smem = tab_bytes;
     }
     SMP_CUDA(cudaMemsetAsync(d_counters, 0, CNT_COUNT * sizeof(unsigned long long), s));

@@ -9,6 +9,8 @@
 // Gap gating (renderer/include/rif_base.h:104-137, cuda_scene.cuh:463-481): outside
 // sgap <= x <= egap the index is n_o and the gradient zero.
 #pragma once
+#include <climits>
+
 #include "dev_math.cuh"
 #include "kparams.h"
 
@@ -23,7 +25,7 @@ static constexpr float kEps = 1.19209290e-07f;    // M_EPSILON (constants.h)
 // cos(m phi), sin(m phi) come from (z/r + i y/r)^m instead of atan2 + sincos.
 // Below r = M_EPSILON the gradient uses y = z = r = M_EPSILON as the reference does.
 template <int M>
-__device__ __forceinline__ void bessel_field_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+__device__ __forceinline__ void bessel_field_any(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
     float y = p.y, z = p.z;
     const float r2 = fmaf(y, y, z * z);
     float rs = rsqrt_fast(r2);                 // +inf at r2 = 0
@@ -75,6 +77,66 @@ __device__ __forceinline__ void bessel_field_ng(const FieldParams &F, const floa
     g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
 }
 
+template <int M>
+static __device__ __noinline__ float4 bessel_field_rare(const FieldParams &F, const float4 *tab, float3 p, float s) {
+    float n;
+    float3 g;
+    bessel_field_any<M>(F, tab, p, s, n, g);
+    return make_float4(g.x, g.y, g.z, n);
+}
+
+// (J_M, J_{M+1}) from the table at the coordinate t = k r / h, with no test on the way: the interval is
+// clamped to the table, and the caller redoes a point whose t is not below bend (or not a number).
+__device__ __forceinline__ void bessel_pair_clamped(const FieldParams &F, const float4 *tab, float t, float &jm, float &jm1) {
+    const float tb = __fadd_rd(t, 8388608.0f);
+    const unsigned i = min(unsigned(__float_as_int(tb) - 0x4B000000), unsigned(F.bint - 1));
+    const float f = t - (tb - 8388608.0f);
+    const float4 a = tab[2 * i], b = tab[2 * i + 1];
+    jm = fmaf(fmaf(fmaf(a.w, f, a.z), f, a.y), f, a.x);
+    jm1 = fmaf(fmaf(fmaf(b.w, f, b.z), f, b.y), f, b.x);
+}
+
+// The same field in one straight line, for the march. A point off the axis and inside the table --
+// practically all of them -- needs no branch; the two tests that find the others are off the step's
+// dependency chain and share one branch at its end. (Each test as a branch of its own before the
+// lookup held the whole chain up until it resolved: the lone tail photon's step took 295 cycles.)
+template <int M>
+__device__ __forceinline__ void bessel_field_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+    const float y = p.y, z = p.z;
+    const float r2 = fmaxf(fmaf(y, y, z * z), 1e-20f);       // a point below is rare anyway: r < kEps
+    const float rs = rsqrt_fast(r2);
+    const float A = F.amp * s;
+    const float r = r2 * rs, t = F.kb * r;
+    float jm, jm1;
+    bessel_pair_clamped(F, tab, t, jm, jm1);
+    if (M == 0) {
+        // grad = A k J_0'(kr) (0, y, z)/r = -A k J_1(kr) (0, y, z)/r
+        n = fmaf(A, jm, F.n_o);
+        const float w = -(A * F.k_r) * jm1 * rs;
+        g = f3(0.0f, w * y, w * z);
+    } else if (M == 1) {
+        // n = n_o + A J_1(kr) z/r; with J_1' = J_1/(kr) - J_2 the gradient reduces to
+        // dn/dy = -A k J_2(kr) y z/r^2,  dn/dz = A J_1(kr)/r - A k J_2(kr) z^2/r^2
+        const float aj = A * jm * rs;
+        n = fmaf(aj, z, F.n_o);
+        const float wz = (A * F.k_r) * jm1 * (rs * rs) * z;
+        g = f3(0.0f, -wz * y, fmaf(-wz, z, aj));
+    } else {
+        const float c = z * rs, sn = y * rs;
+        const float cm = fmaf(c, c, -sn * sn), sm = 2.0f * c * sn;
+        n = fmaf(A * jm, cm, F.n_o);
+        const float djm = fmaf(float(M) * F.inv_k * rs, jm, -jm1);
+        const float a1 = A * djm * F.k_r * rs * cm;
+        const float a2 = A * jm * float(M) * sm * rs * rs;
+        g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
+    }
+    if (!((r >= kEps) & (t < F.bend))) {
+        const float4 q = bessel_field_rare<M>(F, tab, p, s);
+        n = q.w;
+        g = f3(q.x, q.y, q.z);
+    }
+}
+
 // gap gating (rif_base.h:104-137): n_o and no gradient outside sgap <= x <= egap
 __device__ __forceinline__ bool in_gap(const FieldParams &F, float3 p) { return p.x > F.egap || p.x < F.sgap; }
 
@@ -89,7 +151,11 @@ __device__ __forceinline__ void bessel_field(const FieldParams &F, const float4 
 __device__ __forceinline__ void wave_field_ng(const FieldParams &F, float3 p, float tau, float &n, float3 &g) {
     float acc = 0.0f;
     float3 gg = f3(0.0f, 0.0f, 0.0f);
-    for (int i = 0; i < F.n_waves; ++i) {
+    // unrolled, so that every wave's constants are operands of their instructions; with a run-time index
+    // each is a constant-memory load on the step's dependency chain
+#pragma unroll
+    for (int i = 0; i < SMP_MAX_WAVES; ++i) {
+        if (i >= F.n_waves) break;
         float ph = F.wk[i][0] * p.x + F.wk[i][1] * p.y + F.wk[i][2] * p.z - tau + F.wphase[i];
         float sn, cs;
         sincos_red(ph, sn, cs);
@@ -192,90 +258,162 @@ static constexpr int kSplineBrick = 16;
 static constexpr int kSplineBrickRows = kSplineBrick + 3;
 static constexpr int kSplineBrickQuads = kSplineBrick * kSplineBrickRows * kSplineBrickRows;
 
+// One (y, z) row of the 4x4x4 taps: its four x taps times the x weights, into the value and gradient
+// sums. Every spline evaluation adds its sixteen rows through here in the same order.
+struct SplineW { float wx[4], dx[4], wy[4], dy[4], wz[4], dz[4]; };
+struct SplineSum { float v, gx, gy, gz; };
+__device__ __forceinline__ void spline_row(const SplineW &w, int b, int c, float r0, float r1, float r2, float r3,
+                                           SplineSum &s) {
+    const float sv = r0 * w.wx[0] + r1 * w.wx[1] + r2 * w.wx[2] + r3 * w.wx[3];
+    const float sd = r0 * w.dx[0] + r1 * w.dx[1] + r2 * w.dx[2] + r3 * w.dx[3];
+    const float wyz = w.wy[b] * w.wz[c];
+    s.v = fmaf(sv, wyz, s.v);
+    s.gx = fmaf(sd, wyz, s.gx);
+    s.gy = fmaf(sv, w.dy[b] * w.wz[c], s.gy);
+    s.gz = fmaf(sv, w.wy[b] * w.dz[c], s.gz);
+}
+__device__ __forceinline__ void spline_weights(float tx, float ty, float tz, SplineW &w) {
+    bspline_weights(tx, w.wx, w.dx);
+    bspline_weights(ty, w.wy, w.dy);
+    bspline_weights(tz, w.wz, w.dz);
+}
+__device__ __forceinline__ void spline_result(const FieldParams &F, const SplineSum &s, float &n, float3 &g) {
+    n = F.spline_base + s.v;
+    g = f3(s.gx * F.xres[0], s.gy * F.xres[1], s.gz * F.xres[2]);
+}
+
+// The sixteen tap rows of one grid cell, kept in registers while a march stays in it. An ER step
+// is a tenth of a cell or less on the usual grids (0.01 mm steps on 64 to 96 nodes over 10 mm), so
+// a march reads its taps once per cell instead of once per step.
+struct SplineCell {
+    int bx, by, bz;
+    float4 q[16];
+    __device__ __forceinline__ void clear() { bx = by = bz = INT_MIN; }    // no cell starts there
+};
+
+// The rows of the cell whose taps start at (bx, by, bz), sixteen independent 16-byte loads.
+__device__ __forceinline__ void spline_rows(const FieldParams &F, int bx, int by, int bz, float4 q[16]) {
+    const int N0 = F.N[0], N1 = F.N[1], N2 = F.N[2];
+    int iy[4], iz[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        iy[a] = spline_wrap(by + a, N1) * N0;
+        iz[a] = spline_wrap(bz + a, N2) * N0 * N1;
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) q[4 * c + b] = __ldg(F.coeff4 + (iz[c] + iy[b] + bx + 1));
+}
+
+// taps read one by one: a point off the grid in x, or a plan without quads. Returns (grad n, n).
+static __device__ __noinline__ float4 spline_taps(const FieldParams &F, float3 p) {
+    const float tx = (p.x - F.xmin[0]) * F.xres[0], ty = (p.y - F.xmin[1]) * F.xres[1], tz = (p.z - F.xmin[2]) * F.xres[2];
+    SplineW w;
+    spline_weights(tx, ty, tz, w);
+    const int bx = int(floorf(tx)) - 1, by = int(floorf(ty)) - 1, bz = int(floorf(tz)) - 1;
+    const int N0 = F.N[0], N1 = F.N[1], N2 = F.N[2];
+    int ix[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) ix[a] = spline_wrap(bx + a, N0);
+    SplineSum s = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const float *row = F.coeff + spline_wrap(bz + c, N2) * N0 * N1 + spline_wrap(by + b, N1) * N0;
+            spline_row(w, b, c, __ldg(row + ix[0]), __ldg(row + ix[1]), __ldg(row + ix[2]), __ldg(row + ix[3]), s);
+        }
+    float n;
+    float3 g;
+    spline_result(F, s, n, g);
+    return make_float4(g.x, g.y, g.z, n);
+}
+
+__device__ __forceinline__ bool spline_in_gap(const FieldParams &F, float3 p) { return p.x > F.egap || p.x < F.sgap; }
+
+// n and grad n with the taps of the march's current cell kept in C
+__device__ __forceinline__ void spline_field_cell(const FieldParams &F, SplineCell &C, float3 p, float &n, float3 &g) {
+    const float tx = (p.x - F.xmin[0]) * F.xres[0], ty = (p.y - F.xmin[1]) * F.xres[1], tz = (p.z - F.xmin[2]) * F.xres[2];
+    const int bx = int(floorf(tx)) - 1, by = int(floorf(ty)) - 1, bz = int(floorf(tz)) - 1;
+    SplineW w;
+    spline_weights(tx, ty, tz, w);
+    SplineSum s = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (F.coeff4 != nullptr && unsigned(bx + 1) < unsigned(F.N[0])) {
+        if ((bx != C.bx) | (by != C.by) | (bz != C.bz)) {
+            spline_rows(F, bx, by, bz, C.q);
+            C.bx = bx; C.by = by; C.bz = bz;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const float4 q = C.q[4 * c + b];
+                spline_row(w, b, c, q.x, q.y, q.z, q.w, s);
+            }
+    } else {
+        const float4 r = spline_taps(F, p);
+        n = r.w;
+        g = f3(r.x, r.y, r.z);
+        return;
+    }
+    spline_result(F, s, n, g);
+}
+
 __device__ __forceinline__ void spline_field(const FieldParams &F, const float4 *brick, float3 p, float &n, float3 &g) {
-    if (p.x > F.egap || p.x < F.sgap) {
+    if (spline_in_gap(F, p)) {
         n = F.n_o;
         g = f3(0.0f, 0.0f, 0.0f);
         return;
     }
-    float t[3] = {(p.x - F.xmin[0]) * F.xres[0], (p.y - F.xmin[1]) * F.xres[1], (p.z - F.xmin[2]) * F.xres[2]};
-    float wx[4], wy[4], wz[4], dx[4], dy[4], dz[4];
-    bspline_weights(t[0], wx, dx);
-    bspline_weights(t[1], wy, dy);
-    bspline_weights(t[2], wz, dz);
-    int ix[4], iy[4], iz[4];
-    int bx = int(floorf(t[0])) - 1, by = int(floorf(t[1])) - 1, bz = int(floorf(t[2])) - 1;
-    const int N0 = F.N[0], N1 = F.N[1], N2 = F.N[2];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        ix[a] = spline_wrap(bx + a, N0);
-        iy[a] = spline_wrap(by + a, N1) * N0;
-        iz[a] = spline_wrap(bz + a, N2) * N0 * N1;
+    if (brick == nullptr) {
+        SplineCell C;
+        C.clear();
+        spline_field_cell(F, C, p, n, g);
+        return;
     }
-    float v = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
-    // x-tap quads: one 16-byte load per row when floor(t_x) lies on the grid (same values, same
-    // sums as the four single loads)
-    const bool quad = F.coeff4 != nullptr && unsigned(bx + 1) < unsigned(N0);
+    const float tx = (p.x - F.xmin[0]) * F.xres[0], ty = (p.y - F.xmin[1]) * F.xres[1], tz = (p.z - F.xmin[2]) * F.xres[2];
+    SplineW w;
+    spline_weights(tx, ty, tz, w);
+    const int bx = int(floorf(tx)) - 1, by = int(floorf(ty)) - 1, bz = int(floorf(tz)) - 1;
     // the staged brick holds every tap when floor(t) lies in its cells on all three axes (and on
     // the grid)
-    const float4 *bq = nullptr;
-    if (brick != nullptr) {
-        const int4 h = *reinterpret_cast<const int4 *>(brick);
-        const int ox = bx + 1 - h.x, oy = by + 1 - h.y, oz = bz + 1 - h.z;
-        if (h.w != 0 && unsigned(ox) < unsigned(kSplineBrick) && unsigned(oy) < unsigned(kSplineBrick) &&
-            unsigned(oz) < unsigned(kSplineBrick) && unsigned(bx + 1) < unsigned(N0) && unsigned(by + 1) < unsigned(N1) &&
-            unsigned(bz + 1) < unsigned(N2))
-            bq = brick + 1 + (oz * kSplineBrickRows + oy) * kSplineBrick + ox;
-    }
+    const int4 h = *reinterpret_cast<const int4 *>(brick);
+    const int ox = bx + 1 - h.x, oy = by + 1 - h.y, oz = bz + 1 - h.z;
+    SplineSum s = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (h.w != 0 && unsigned(ox) < unsigned(kSplineBrick) && unsigned(oy) < unsigned(kSplineBrick) &&
+        unsigned(oz) < unsigned(kSplineBrick) && unsigned(bx + 1) < unsigned(F.N[0]) && unsigned(by + 1) < unsigned(F.N[1]) &&
+        unsigned(bz + 1) < unsigned(F.N[2])) {
+        const float4 *bq = brick + 1 + (oz * kSplineBrickRows + oy) * kSplineBrick + ox;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            float r0, r1, r2, r3;
-            if (bq != nullptr) {
+            for (int b = 0; b < 4; ++b) {
                 const float4 q = bq[(c * kSplineBrickRows + b) * kSplineBrick];
-                r0 = q.x; r1 = q.y; r2 = q.z; r3 = q.w;
-            } else if (quad) {
-                const float4 q = __ldg(F.coeff4 + (iz[c] + iy[b] + bx + 1));
-                r0 = q.x; r1 = q.y; r2 = q.z; r3 = q.w;
-            } else {
-                const float *row = F.coeff + iz[c] + iy[b];
-                r0 = __ldg(row + ix[0]); r1 = __ldg(row + ix[1]); r2 = __ldg(row + ix[2]); r3 = __ldg(row + ix[3]);
+                spline_row(w, b, c, q.x, q.y, q.z, q.w, s);
             }
-            float sv = r0 * wx[0] + r1 * wx[1] + r2 * wx[2] + r3 * wx[3];
-            float sd = r0 * dx[0] + r1 * dx[1] + r2 * dx[2] + r3 * dx[3];
-            float wyz = wy[b] * wz[c];
-            v = fmaf(sv, wyz, v);
-            gx = fmaf(sd, wyz, gx);
-            gy = fmaf(sv, dy[b] * wz[c], gy);
-            gz = fmaf(sv, wy[b] * dz[c], gz);
-        }
+    } else if (F.coeff4 != nullptr && unsigned(bx + 1) < unsigned(F.N[0])) {
+        float4 q[16];
+        spline_rows(F, bx, by, bz, q);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) spline_row(w, b, c, q[4 * c + b].x, q[4 * c + b].y, q[4 * c + b].z, q[4 * c + b].w, s);
+    } else {
+        const float4 r = spline_taps(F, p);
+        n = r.w;
+        g = f3(r.x, r.y, r.z);
+        return;
     }
-    n = F.spline_base + v;
-    g = f3(gx * F.xres[0], gy * F.xres[1], gz * F.xres[2]);
+    spline_result(F, s, n, g);
 }
 
-// Field<FK>::eval(F, tab, p, s, n, g): tab is the Bessel table (shared memory in the march
-// kernel), unused by the other kinds.
-template <int FK> struct Field;
-template <> struct Field<FK_BESSEL0> {
-    static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) { bessel_field<0>(F, tab, p, s, n, g); }
-    static __device__ __forceinline__ void eval_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) { bessel_field_ng<0>(F, tab, p, s, n, g); }
-};
-template <> struct Field<FK_BESSEL1> {
-    static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) { bessel_field<1>(F, tab, p, s, n, g); }
-    static __device__ __forceinline__ void eval_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) { bessel_field_ng<1>(F, tab, p, s, n, g); }
-};
-template <> struct Field<FK_BESSEL2> {
-    static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) { bessel_field<2>(F, tab, p, s, n, g); }
-    static __device__ __forceinline__ void eval_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) { bessel_field_ng<2>(F, tab, p, s, n, g); }
-};
 // Bessel mode m in 0..2 chosen at run time, one branch-free path for all orders (lanes of a warp
 // may hold photons of different instances and orders): cos/sin(m phi) by selects from
 // (z + iy)/r, J_m' = (m/kr) J_m - J_{m+1}; beyond the table the order-specific formulas.
-__device__ __forceinline__ void bessel_field_rt(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+__device__ __forceinline__ void bessel_field_rt_any(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
     const int M = F.mode;
-    const float A = F.amp * (in_gap(F, p) ? 0.0f : s);
+    const float A = F.amp * s;
     float y = p.y, z = p.z;
     const float r2 = fmaf(y, y, z * z);
     float rs = rsqrt_fast(r2);                 // +inf at r2 = 0
@@ -315,14 +453,45 @@ __device__ __forceinline__ void bessel_field_rt(const FieldParams &F, const floa
     const float a2 = A * jm * fm * sm * rs * rs;
     g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
 }
+static __device__ __noinline__ float4 bessel_field_rt_rare(const FieldParams &F, const float4 *tab, float3 p, float s) {
+    float n;
+    float3 g;
+    bessel_field_rt_any(F, tab, p, s, n, g);
+    return make_float4(g.x, g.y, g.z, n);
+}
+// in one straight line, as bessel_field_ng
+__device__ __forceinline__ void bessel_field_rt_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+    const int M = F.mode;
+    const float A = F.amp * s;
+    const float y = p.y, z = p.z;
+    const float r2 = fmaxf(fmaf(y, y, z * z), 1e-20f);
+    const float rs = rsqrt_fast(r2);
+    const float r = r2 * rs, t = F.kb * r;
+    const float c = z * rs, sn = y * rs;
+    const float cm = M == 0 ? 1.0f : (M == 1 ? c : fmaf(c, c, -sn * sn));
+    const float sm = M == 0 ? 0.0f : (M == 1 ? sn : 2.0f * c * sn);
+    float jm, jm1;
+    bessel_pair_clamped(F, tab, t, jm, jm1);
+    n = fmaf(A * jm, cm, F.n_o);
+    const float fm = float(M);
+    const float djm = fmaf(fm * F.inv_k * rs, jm, -jm1);
+    const float a1 = A * djm * F.k_r * rs * cm;
+    const float a2 = A * jm * fm * sm * rs * rs;
+    g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
+    if (!((r >= kEps) & (t < F.bend))) {
+        const float4 q = bessel_field_rt_rare(F, tab, p, s);
+        n = q.w;
+        g = f3(q.x, q.y, q.z);
+    }
+}
 
 // Bessel mode m >= 3 (scene.cpp:206-257 take any integer order through jn(mode, .)): J_m and J_m+1
 // from the per-plan table, which the host sizes to cover the whole box (k r <= 128, checked when the
 // plan is made; a point beyond it reads the table's last interval); cos(m phi), sin(m phi) as
 // ((z + i y)/r)^m by m - 1 complex products.
-__device__ __forceinline__ void bessel_field_n(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+__device__ __forceinline__ void bessel_field_n_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
     const int M = F.mode;
-    const float A = F.amp * (in_gap(F, p) ? 0.0f : s);
+    const float A = F.amp * s;
     float y = p.y, z = p.z;
     const float r2 = fmaf(y, y, z * z);
     float rs = rsqrt_fast(r2);                 // +inf at r2 = 0
@@ -359,36 +528,68 @@ __device__ __forceinline__ void bessel_field_n(const FieldParams &F, const float
     const float a2 = A * jm * fm * sm * rs * rs;
     g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
 }
-template <> struct Field<FK_BESSELN> {
-    static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
-        bessel_field_n(F, tab, p, s, n, g);
+// Field<FK>: the field of one kind. tab is the Bessel table (shared memory in the march kernel) or
+// the staged spline brick, unused by the other kinds.
+//   eval(F, tab, p, s, n, g)          n and grad n at p
+//   eval_c(F, tab, C, p, s, n, g)     the same, with what the march carries from step to step in C
+//   eval_in(F, tab, C, p, s, n, g)    the same for a p known to lie in the field (not in a gap)
+// All three give the same bits at the same point.
+struct NoCache {
+    __device__ __forceinline__ void clear() {}
+};
+template <int FK> struct Field;
+#define SMP_FIELD(FK, IN, ALL)                                                                                      \
+    template <> struct Field<FK> {                                                                                  \
+        using Cache = NoCache;                                                                                      \
+        static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) { ALL; } \
+        static __device__ __forceinline__ void eval_c(const FieldParams &F, const float4 *tab, Cache &, float3 p, float s, float &n, float3 &g) { ALL; } \
+        static __device__ __forceinline__ void eval_in(const FieldParams &F, const float4 *tab, Cache &, float3 p, float s, float &n, float3 &g) { IN; } \
+    };
+SMP_FIELD(FK_BESSEL0, bessel_field_ng<0>(F, tab, p, s, n, g), bessel_field<0>(F, tab, p, s, n, g))
+SMP_FIELD(FK_BESSEL1, bessel_field_ng<1>(F, tab, p, s, n, g), bessel_field<1>(F, tab, p, s, n, g))
+SMP_FIELD(FK_BESSEL2, bessel_field_ng<2>(F, tab, p, s, n, g), bessel_field<2>(F, tab, p, s, n, g))
+SMP_FIELD(FK_BESSELN, bessel_field_n_ng(F, tab, p, s, n, g), bessel_field_n_ng(F, tab, p, in_gap(F, p) ? 0.0f : s, n, g))
+// batched sweep: the instance's Bessel field
+SMP_FIELD(FK_BATCH, bessel_field_rt_ng(F, tab, p, s, n, g), bessel_field_rt_ng(F, tab, p, in_gap(F, p) ? 0.0f : s, n, g))
+SMP_FIELD(FK_PLANEWAVE, wave_field_ng(F, p, s, n, g), wave_field(F, p, s, n, g))
+SMP_FIELD(FK_SOURCES, sources_field(F, p, n, g), sources_field(F, p, n, g))
+#undef SMP_FIELD
+// The field at a start point, for the discrete logic between marches: the spline's sixteen rows are
+// kept out of its registers by a call.
+template <int FK>
+__device__ __forceinline__ void field_at(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+    Field<FK>::eval(F, tab, p, s, n, g);
+}
+template <> struct Field<FK_SPLINE> {
+    using Cache = SplineCell;
+    // inlined only where a step of the brick kernel needs it; the discrete logic calls it
+    static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *brick, float3 p, float, float &n, float3 &g) {
+        spline_field(F, brick, p, n, g);
     }
-    static __device__ __forceinline__ void eval_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
-        bessel_field_n(F, tab, p, s, n, g);
+    static __device__ __noinline__ float4 eval_call(const FieldParams &F, float3 p) {
+        float n;
+        float3 g;
+        spline_field(F, nullptr, p, n, g);
+        return make_float4(g.x, g.y, g.z, n);
+    }
+    static __device__ __forceinline__ void eval_c(const FieldParams &F, const float4 *, Cache &C, float3 p, float, float &n, float3 &g) {
+        if (spline_in_gap(F, p)) {
+            n = F.n_o;
+            g = f3(0.0f, 0.0f, 0.0f);
+            return;
+        }
+        spline_field_cell(F, C, p, n, g);
+    }
+    static __device__ __forceinline__ void eval_in(const FieldParams &F, const float4 *, Cache &C, float3 p, float, float &n, float3 &g) {
+        spline_field_cell(F, C, p, n, g);
     }
 };
 
-// batched sweep: the instance's Bessel field
-template <> struct Field<FK_BATCH> {
-    static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
-        bessel_field_rt(F, tab, p, s, n, g);
-    }
-    static __device__ __forceinline__ void eval_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
-        bessel_field_rt(F, tab, p, s, n, g);
-    }
-};
-template <> struct Field<FK_PLANEWAVE> {
-    static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *, float3 p, float s, float &n, float3 &g) { wave_field(F, p, s, n, g); }
-    static __device__ __forceinline__ void eval_ng(const FieldParams &F, const float4 *, float3 p, float s, float &n, float3 &g) { wave_field_ng(F, p, s, n, g); }
-};
-template <> struct Field<FK_SOURCES> {
-    static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *, float3 p, float, float &n, float3 &g) { sources_field(F, p, n, g); }
-    static __device__ __forceinline__ void eval_ng(const FieldParams &F, const float4 *, float3 p, float, float &n, float3 &g) { sources_field(F, p, n, g); }
-};
-// the spline's `tab` argument is the staged brick of the slot pool's march kernel (or nullptr)
-template <> struct Field<FK_SPLINE> {
-    static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *brick, float3 p, float, float &n, float3 &g) { spline_field(F, brick, p, n, g); }
-    static __device__ __forceinline__ void eval_ng(const FieldParams &F, const float4 *brick, float3 p, float, float &n, float3 &g) { spline_field(F, brick, p, n, g); }
-};
+template <>
+__device__ __forceinline__ void field_at<FK_SPLINE>(const FieldParams &F, const float4 *, float3 p, float, float &n, float3 &g) {
+    const float4 r = Field<FK_SPLINE>::eval_call(F, p);
+    n = r.w;
+    g = f3(r.x, r.y, r.z);
+}
 
 }  // namespace smp

@@ -51,9 +51,12 @@ struct FieldParams {
     // J_m+1 in f = x/bh - i; bint intervals, bnodes = 2 * bint float4 entries
     const float4 *btab;
     int bnodes, bint;
+    float bend;             // float(bint)
     float bh, binv_h;
     float kb;               // k_r / bh: table coordinate per metre of r
-    float grad_bound;       // bound on |grad n|_1 anywhere (0: unknown)
+    // bounds for the march's untested windows (march.cuh safe_steps): |grad n|_1 <= grad_bound and
+    // n >= n_low anywhere in the field; n_low = 0: no bounds, every step is tested
+    float grad_bound, n_low;
 };
 
 #define SMP_MAX_REFINE 39
@@ -77,6 +80,9 @@ struct KParams {
     float L[3], R[3];
     // the same box as exact float thresholds: p - L > -eps  <=>  p >= box_lo, R - p > -eps  <=>  p <= box_hi
     float box_lo[3], box_hi[3];
+    // untested windows (march.cuh safe_steps): the shortest step they take, 6e-6 of the box's largest
+    // coordinate, and that coordinate's rounding, 2^-23 of it
+    float win_hmin, win_round;
     // textured source (area_textured_source)
     float src_origin[3];
     float plane[2], pixsize[2];
@@ -122,6 +128,8 @@ struct KParams {
     const long long *offsets;
     // work: photons [first_photon, first_photon + n_photons)
     long long first_photon, n_photons;
+    long long fetch_from;             // photons below it start in a lane of their own (wf_finish_kernel);
+                                      // the counter hands out the rest
     unsigned long long *counters;     // device scratch, see Counter
     smp_photon_record *records;       // trace mode only (indexed by photon - first_photon)
     int event_batch;                  // lanes that must finish a march before the warp runs events

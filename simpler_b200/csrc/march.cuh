@@ -16,6 +16,9 @@
 #include <cooperative_groups.h>
 #include <cooperative_groups/reduce.h>
 
+#include <climits>
+#include <type_traits>
+
 #include "dev_field.cuh"
 #include "kparams.h"
 
@@ -30,6 +33,8 @@ static constexpr unsigned kFull = 0xffffffffu;
 #ifndef SMP_MIN_BLOCKS
 #define SMP_MIN_BLOCKS 4
 #endif
+// The spline's lane loops hold the 64 taps of a cell in registers: two blocks.
+constexpr int lane_blocks(int fk) { return fk == FK_SPLINE ? 2 : SMP_MIN_BLOCKS; }
 
 enum LaneState : int { ST_FETCH = 0, ST_EVENT = 1, ST_MARCH = 2, ST_DONE = 3, ST_HOOK = 4 };
 enum Event : int {
@@ -376,7 +381,7 @@ __device__ __forceinline__ const float *step_tab(const S &L, const KParams &P) {
 
 template <int FK>
 __device__ __forceinline__ void begin_march(Lane &L, const KParams &P, float dlimit, bool eval) {
-    if (eval) Field<FK>::eval(field_of<FK>(L, P), L.tab, L.mp, L.s, L.mn, L.mg);
+    if (eval) field_at<FK>(field_of<FK>(L, P), L.tab, L.mp, L.s, L.mn, L.mg);
     const float h0 = step_h0<FK>(L, P);
     L.dist_acc = 0.0f;
     L.dlimit = dlimit;
@@ -399,15 +404,19 @@ __device__ __forceinline__ bool march_has_steps(const Lane &L) { return L.stop >
 // (thresholds box_lo/box_hi, exact) and the distance test (dist_acc + cur <= dlimit) are one chain
 // of predicate comparisons, and the loop count and the step cap share one counter (`stop` is the
 // loop's end clamped to the cap; the cap is told apart on the rare path).
-template <int FK, int FP = -1, class S>
-__device__ __forceinline__ bool march_step(S &L, const KParams &P) {
+//
+// C carries what the field keeps from step to step (Field<FK>::Cache), or is a NoCache: the field is
+// then evaluated through L.tab alone (the staged spline brick).
+template <int FK, int FP = -1, class S, class CA>
+__device__ __forceinline__ bool march_step(S &L, const KParams &P, CA &C) {
     const bool f64 = FP < 0 ? P.fp64 != 0 : FP != 0;     // FP: the path-length form, if fixed at compile time
     const float3 d = f3(fmaf(L.hh, L.mg.x, L.md.x), fmaf(L.hh, L.mg.y, L.md.y), fmaf(L.hh, L.mg.z, L.md.z));
     const float hinv = L.cur * rcp_fast(L.mn);
     const float3 p = f3(fmaf(d.x, hinv, L.mp.x), fmaf(d.y, hinv, L.mp.y), fmaf(d.z, hinv, L.mp.z));
     float n2;
     float3 g2;
-    Field<FK>::eval(field_of<FK>(L, P), L.tab, p, L.s, n2, g2);
+    if constexpr (std::is_same<CA, NoCache>::value) Field<FK>::eval(field_of<FK>(L, P), L.tab, p, L.s, n2, g2);
+    else Field<FK>::eval_c(field_of<FK>(L, P), L.tab, C, p, L.s, n2, g2);
     const float3 d2 = f3(fmaf(L.hh, g2.x, d.x), fmaf(L.hh, g2.y, d.y), fmaf(L.hh, g2.z, d.z));
     ++L.steps;
     const float sacc = L.dist_acc + L.cur;
@@ -443,6 +452,64 @@ __device__ __forceinline__ bool march_step(S &L, const KParams &P) {
     return false;
 }
 
+// ---- untested windows -------------------------------------------------------------------------
+// A step's tests (seven comparisons in a chain, the loop count, the branch they feed) come after its
+// position, and the next step waits for their branch: one photon alone in its warp took 440 cycles a
+// step, three times the arithmetic's own chain. Far from a face and from the sampled distance none
+// of them can fail, so a lane that marches alone, or with few others, runs windows: the number of
+// steps that provably pass every test is worked out once, and those steps run without them. The
+// steps' arithmetic is march_step's own, so the photon is the same bit for bit.
+//
+// safe_steps: a lower bound on the steps, at most `cap`, that pass every test of march_step from
+// here (<= 0: none known). A step moves a coordinate by at most h |d_a| / n, where n >= n_low and the
+// momentum component d_a changes by at most h grad_bound a step; 3 % and 3e-7 a step cover the
+// rounding of the momentum, the reciprocal and this bound itself, win_round the position's. The path
+// distance gains h a step, and the rounding of its sum. The x range is the field's, inside the gaps.
+template <int FK, class S>
+__device__ __forceinline__ int safe_steps(const S &L, const KParams &P, int cap) {
+    const FieldParams &F = field_of<FK>(L, P);
+    const float h = L.cur;
+    if (!(F.n_low > 0.0f) || !(h >= P.win_hmin)) return 0;
+    const float kick = fmaf(F.grad_bound, h, 3e-7f) * float(cap + 1);
+    const float q = __fdividef(1.03f * h, F.n_low);
+    const float mx = fminf(L.mp.x - fmaxf(P.box_lo[0], F.sgap), fminf(P.box_hi[0], F.egap) - L.mp.x);
+    const float my = fminf(L.mp.y - P.box_lo[1], P.box_hi[1] - L.mp.y);
+    const float mz = fminf(L.mp.z - P.box_lo[2], P.box_hi[2] - L.mp.z);
+    const float kx = __fdividef(mx, fmaf(q, fabsf(L.md.x) + kick, P.win_round));
+    const float ky = __fdividef(my, fmaf(q, fabsf(L.md.y) + kick, P.win_round));
+    const float kz = __fdividef(mz, fmaf(q, fabsf(L.md.z) + kick, P.win_round));
+    const float kd = __fdividef(L.dlimit - L.dist_acc, fmaf(1.03f, h, 1.2e-7f * L.dlimit));
+    const float k = 0.999f * fminf(fminf(kx, ky), fminf(kz, kd));
+    if (!(k >= 1.0f)) return 0;                            // no room, or not a number
+    return min(int(fminf(k, float(cap))), L.stop - L.steps - 1);
+}
+
+// `k` steps of march_step that safe_steps has shown to be accepted
+template <int FK, class S>
+__device__ __forceinline__ void march_window(S &L, const KParams &P, int k, typename Field<FK>::Cache &C) {
+    const FieldParams &F = field_of<FK>(L, P);
+    const float h = L.cur, hh = L.hh, s = L.s;
+    const double hd = L.cur_d;
+    const bool f64 = P.fp64 != 0;
+    float3 p = L.mp, v = L.md, g = L.mg;
+    float n = L.mn, acc = L.dist_acc, totf = L.mtotf;
+    double tot = L.mtot;
+#pragma unroll 1
+    for (int i = 0; i < k; ++i) {
+        const float3 d = f3(fmaf(hh, g.x, v.x), fmaf(hh, g.y, v.y), fmaf(hh, g.z, v.z));
+        const float hinv = h * rcp_fast(n);
+        p = f3(fmaf(d.x, hinv, p.x), fmaf(d.y, hinv, p.y), fmaf(d.z, hinv, p.z));
+        Field<FK>::eval_in(F, L.tab, C, p, s, n, g);
+        v = f3(fmaf(hh, g.x, d.x), fmaf(hh, g.y, d.y), fmaf(hh, g.z, d.z));
+        acc = acc + h;
+        if (f64) tot = fma(hd, double(n), tot);
+        else totf = fmaf(h, n, totf);
+    }
+    L.mp = p; L.md = v; L.mg = g; L.mn = n;
+    L.dist_acc = acc; L.mtotf = totf; L.mtot = tot;
+    L.steps += k;
+}
+
 // ---- discrete logic between marches ---------------------------------------------------------
 // Observation points for path replay (adjoint.cuh). The render kernels use NoHook, for which every
 // hook call below is compiled out.
@@ -453,7 +520,7 @@ struct NoHook {
     __device__ void photon_begin(const Lane &) {}
     __device__ void photon_end(const Lane &) {}
     __device__ void march_begin() {}
-    __device__ void accepted() {}
+    __device__ void accepted(int) {}
 };
 
 // Runs the lane's events until it starts a march (returns ST_MARCH) or its photon ends
@@ -507,7 +574,7 @@ __device__ __forceinline__ int run_events(Lane &L, const KParams &P, int ev, H *
                 L.s = fmaxf(fminf(sn, F.max_scaling), -F.max_scaling);
             }
             L.mp = L.pos;
-            Field<FK>::eval(F, L.tab, L.mp, L.s, L.mn, L.mg);
+            field_at<FK>(F, L.tab, L.mp, L.s, L.mn, L.mg);
             L.dir = mul(L.dir, L.mn);                     // photon.cpp:329
             if (P.use_direct) {
                 L.ctx = CTX_DIRECT;
@@ -776,7 +843,7 @@ __device__ __forceinline__ void lane_loop(Lane &L, int st, const KParams &P, Lan
                 if (lane == leader) base = atomicAdd(P.counters + CNT_NEXT_PHOTON, (unsigned long long)__popc(need));
                 base = __shfl_sync(kFull, base, leader);
                 if (st == ST_FETCH) {
-                    unsigned long long k = base + __popc(need & ((1u << lane) - 1u));
+                    unsigned long long k = base + __popc(need & ((1u << lane) - 1u)) + (unsigned long long)P.fetch_from;
                     if (k < (unsigned long long)P.n_photons) {
                         L.idx = P.first_photon + (long long)k;
                         L.end = 0;                       // the previous photon's end code
@@ -801,20 +868,29 @@ __device__ __forceinline__ void lane_loop(Lane &L, int st, const KParams &P, Lan
         const unsigned alive = __ballot_sync(kFull, st != ST_DONE);
         if (alive == 0) break;
         const int thr = max(1, (P.event_batch * __popc(alive) + 16) >> 5);
+        // a lane alone in its warp takes long windows; lanes together take short ones, so that none
+        // waits long for another's
+        const int wcap = (alive & (alive - 1u)) == 0u ? 1024 : 32;
+        typename Field<FK>::Cache C;
+        C.clear();
         for (;;) {
-            // two steps per vote; a lane whose march ends on the first skips the second
-            if (!H::on) {
-                if (st == ST_MARCH && (march_step<FK>(L, P) || march_step<FK>(L, P))) {
+            if (st == ST_MARCH) {
+                bool end = false;
+                const int w = FK == FK_SOURCES ? 0 : safe_steps<FK>(L, P, wcap);
+                if (w >= 4) {
+                    march_window<FK>(L, P, w, C);
+                    if (H::on) h->accepted(w);
+                } else {
+#pragma unroll 1
+                    for (int t = 0; t < (FK == FK_SOURCES ? 2 : 8) && !end; ++t) {
+                        const float3 q = L.mp;
+                        end = march_step<FK>(L, P, C);
+                        if (H::on && (q.x != L.mp.x || q.y != L.mp.y || q.z != L.mp.z)) h->accepted(1);
+                    }
+                }
+                if (end) {
                     st = ST_EVENT;
                     pending_ev = EV_MARCH_END;
-                }
-            } else if (st == ST_MARCH) {
-                // the same two steps, telling the hook which ones were accepted
-                for (int t = 0; t < 2; ++t) {
-                    const float3 q = L.mp;
-                    const bool end = march_step<FK>(L, P);
-                    if (q.x != L.mp.x || q.y != L.mp.y || q.z != L.mp.z) h->accepted();
-                    if (end) { st = ST_EVENT; pending_ev = EV_MARCH_END; break; }
                 }
             }
             const unsigned waiting = __ballot_sync(kFull, st == ST_EVENT);
@@ -845,7 +921,7 @@ __device__ __forceinline__ void flush_stats(LaneStats &S, const KParams &P, int 
 }
 
 template <int FK>
-__global__ void __launch_bounds__(128, SMP_MIN_BLOCKS) march_kernel(const __grid_constant__ KParams P) {
+__global__ void __launch_bounds__(128, lane_blocks(FK)) march_kernel(const __grid_constant__ KParams P) {
     extern __shared__ __align__(16) float4 smem_tab[];
     const int lane = threadIdx.x & 31;
     Lane L;

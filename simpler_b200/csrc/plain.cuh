@@ -28,7 +28,9 @@ __global__ void __launch_bounds__(kPlainBlock) plain_kernel(const __grid_constan
         L.tab = P.field.btab;                 // the Bessel table read from global memory
         int st = run_events<FK>(L, P, EV_NEW);
         while (st == ST_MARCH) {
-            while (!march_step<FK>(L, P)) {
+            typename Field<FK>::Cache C;
+            C.clear();
+            while (!march_step<FK>(L, P, C)) {
             }
             st = run_events<FK>(L, P, EV_MARCH_END);
         }

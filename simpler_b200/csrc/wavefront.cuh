@@ -239,7 +239,7 @@ __device__ __forceinline__ void warp_append2(int *arr, unsigned *c, int n_slots,
 // are not paced by launch latency. F64: the FP64 path-length form (only its accumulator is
 // loaded, carried and stored).
 template <int FK, int F64, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, (FK == FK_SPLINE ? 4 : SMP_WF_MARCH_MIN_BLOCKS) * 128 / BLOCK)
+__global__ void __launch_bounds__(BLOCK, (FK == FK_SPLINE ? 3 : SMP_WF_MARCH_MIN_BLOCKS) * 128 / BLOCK)
 wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveParams W, int it) {
     extern __shared__ __align__(16) float4 smem_tab[];
     const int lane = threadIdx.x & 31, cur = it & 1, nxt = cur ^ 1;
@@ -282,8 +282,10 @@ wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveP
                 M.tab = FK == FK_SPLINE ? nullptr : smem_tab;   // no staged brick: global quads
             }
             const int steps0 = M.steps;
+            typename Field<FK>::Cache C;
+            C.clear();
             for (int k = 0; k < chunk; k += 2) {
-                if (march_step<FK, F64>(M, P) || march_step<FK, F64>(M, P)) { ended = true; break; }
+                if (march_step<FK, F64>(M, P, C) || march_step<FK, F64>(M, P, C)) { ended = true; break; }
             }
             done += unsigned(M.steps - steps0);
             W.ma[slot] = make_float4(M.mp.x, M.mp.y, M.mp.z, M.mn);
@@ -429,8 +431,9 @@ wf_march_spline_kernel(const __grid_constant__ KParams P, const __grid_constant_
             M.tab = brick;
             M.inst = nullptr;
             const int steps0 = M.steps;
+            NoCache C;                               // the taps come from the staged brick
             for (int k = 0; k < chunk; k += 2) {
-                if (march_step<FK_SPLINE, F64>(M, P) || march_step<FK_SPLINE, F64>(M, P)) { ended = true; break; }
+                if (march_step<FK_SPLINE, F64>(M, P, C) || march_step<FK_SPLINE, F64>(M, P, C)) { ended = true; break; }
             }
             done += unsigned(M.steps - steps0);
             W.ma[slot] = make_float4(M.mp.x, M.mp.y, M.mp.z, M.mn);
@@ -522,31 +525,48 @@ wf_event_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveP
     flush_stats(S, P, lane);
 }
 
-// The tail: once the photon counter is exhausted the live slots drain, and a march launch lasts
-// as long as its longest march while slots with short marches wait for the next event launch. When
-// the live slots fit in one persistent grid, this kernel loads each into a lane of the persistent
-// loop (march and events in one kernel, march.cuh) and runs them to the end. A grid too small for
-// the list is a host error, recorded in CNT_LOST.
+// The tail, and small renders as a whole. Once the photon counter is exhausted the live slots drain,
+// and a march launch lasts as long as its longest march while slots with short marches wait for the
+// next event launch. When the live slots fit in one persistent grid, this kernel loads each into a
+// lane of the persistent loop (march and events in one kernel, march.cuh) and runs them to the end.
+// With it < 0 (a render of few photons) there is no pool: lane j starts photon j < fetch_from and the
+// counter hands out the rest.
+//
+// Both end with the longest photon marching alone -- about 1e5 steps of an internally reflected
+// connection, whatever the photon count -- so what bounds them is one photon's chain of steps, and the
+// photons are spread over the warps, block after block, warp after warp, before a second one shares a
+// warp: a lane whose warp holds no other marches in long untested windows and waits for nobody's events.
+// A grid too small for the list is a host error, recorded in CNT_LOST.
 template <int FK>
-__global__ void __launch_bounds__(128, SMP_MIN_BLOCKS)
+__global__ void __launch_bounds__(128, lane_blocks(FK))
 wf_finish_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveParams W, int it) {
     extern __shared__ __align__(16) float4 smem_tab[];
     const int lane = threadIdx.x & 31, cur = it & 1;
-    const unsigned n0 = list_cnt(W, cur)[0], n = n0 + list_cnt(W, cur)[1];
-    const unsigned gid = blockIdx.x * blockDim.x + threadIdx.x, lanes = gridDim.x * blockDim.x;
-    if (gid == 0 && n > lanes) atomicAdd(P.counters + CNT_LOST, (unsigned long long)(n - lanes));
+    const bool direct = it < 0;
+    const unsigned n0 = direct ? 0u : list_cnt(W, cur)[0], n = direct ? 0u : n0 + list_cnt(W, cur)[1];
+    const unsigned lanes = gridDim.x * blockDim.x;
+    const unsigned j = (unsigned(lane) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * gridDim.x + blockIdx.x;
+    if (j == 0 && n > lanes) atomicAdd(P.counters + CNT_LOST, (unsigned long long)(n - lanes));
     const float4 *tab = P.field.btab;
-    if (FK <= FK_BESSELN && P.field.btab != nullptr) {
-        if (stage_to_shared(smem_tab, P.field.btab, unsigned(P.field.bnodes) * 16u, P.counters + CNT_STAGE_TIMEOUT))
-            tab = smem_tab;
+    if (FK <= FK_BESSELN) {                          // always in shared memory, so that the lookups are shared loads
+        if (!stage_to_shared(smem_tab, P.field.btab, unsigned(P.field.bnodes) * 16u, P.counters + CNT_STAGE_TIMEOUT)) {
+            for (int i = threadIdx.x; i < P.field.bnodes; i += blockDim.x) smem_tab[i] = P.field.btab[i];
+            __syncthreads();
+        }
+        tab = smem_tab;
     }
     Lane L;
     L.end = 0;
     L.idx = 0;
     int st = ST_FETCH;
     L.inst = nullptr;
-    if (gid < n) {
-        wf_load_lane(W, P, (FK == FK_SPLINE && W.nb) ? brick_slot(W, cur, gid) : two_class_at(W.list[cur], n0, W.n_slots, gid), L);
+    if (direct) {
+        if ((long long)j < P.fetch_from) {
+            L.idx = P.first_photon + (long long)j;
+            st = ST_EVENT;                           // lane_loop starts it (EV_NEW)
+        }
+    } else if (j < n) {
+        wf_load_lane(W, P, (FK == FK_SPLINE && W.nb) ? brick_slot(W, cur, j) : two_class_at(W.list[cur], n0, W.n_slots, j), L);
         st = ST_MARCH;
     }
     L.tab = (FK == FK_BATCH && L.inst) ? L.inst->field.btab : tab;
