@@ -368,13 +368,19 @@ template <> struct FieldAdj<FK_SPLINE> {
         float hxx = 0.0f, hyy = 0.0f, hzz = 0.0f, hxy = 0.0f, hxz = 0.0f, hyz = 0.0f;
         const int fx = int(floorf((p.x - F.xmin[0]) * F.xres[0]));
         const bool quad = F.coeff4 != nullptr && unsigned(fx) < unsigned(F.N[0]);
+        int ry[4], rz[4];                                   // the quads' rows
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            ry[q] = iy[q] + 2 * spline_wrap(int(floorf((p.y - F.xmin[1]) * F.xres[1])) - 1 + q, F.N[1]);
+            rz[q] = iz[q] + 2 * F.N[1] * spline_wrap(int(floorf((p.z - F.xmin[2]) * F.xres[2])) - 1 + q, F.N[2]);
+        }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 float r0, r1, r2, r3;
                 if (quad) {
-                    const float4 q = __ldg(F.coeff4 + (iz[c] + iy[b] + fx));
+                    const float4 q = __ldg(F.coeff4 + (rz[c] + ry[b] + fx));
                     r0 = q.x; r1 = q.y; r2 = q.z; r3 = q.w;
                 } else {
                     const float *row = F.coeff + iz[c] + iy[b];

@@ -158,14 +158,17 @@ static int spline_mirror(int i, int n) {
     return w >= n ? m - w : w;
 }
 static void spline_quads(const int N[3], const std::vector<float> &delta, std::vector<float4> &quads) {
-    const size_t rows = size_t(N[1]) * N[2];
-    quads.resize(rows * N[0]);
-    for (size_t r = 0; r < rows; ++r)
-        for (int x = 0; x < N[0]; ++x) {
-            const float *row = delta.data() + r * N[0];
-            quads[r * N[0] + x] = make_float4(row[spline_mirror(x - 1, N[0])], row[x], row[spline_mirror(x + 1, N[0])],
-                                              row[spline_mirror(x + 2, N[0])]);
+    const size_t rows = size_t(N[1]) * N[2], stride = size_t(N[0]) + 2;
+    quads.resize(rows * stride);
+    for (size_t r = 0; r < rows; ++r) {
+        const float *row = delta.data() + r * N[0];
+        float4 *out = quads.data() + r * stride + 1;
+        for (int x = -1; x <= N[0]; ++x) {
+            if (x >= 1 && x < N[0] - 2) out[x] = make_float4(row[x - 1], row[x], row[x + 1], row[x + 2]);
+            else out[x] = make_float4(row[spline_mirror(x - 1, N[0])], row[spline_mirror(x, N[0])],
+                                      row[spline_mirror(x + 1, N[0])], row[spline_mirror(x + 2, N[0])]);
         }
+    }
 }
 
 // The quads again with their rows padded for the brick march kernel (dev_field.cuh kSplineBrick): row
@@ -629,7 +632,8 @@ static int plan_setup_field(smp_plan *p, const smp_field_desc &f) {
         p->d_coeff4 = nullptr;
         SMP_CUDA(cudaMalloc(&p->d_coeff4, quads.size() * sizeof(float4)));
         SMP_CUDA(cudaMemcpy(p->d_coeff4, quads.data(), quads.size() * sizeof(float4), cudaMemcpyHostToDevice));
-        p->kp.field.coeff4 = p->d_coeff4;
+        p->kp.field.coeff4 = p->d_coeff4 + 1;              // entry x = 0 of the first row
+        p->kp.field.qrow = f.grid_n[0] + 2;
         // bricks for the slot pool's march kernel (opts.spline_bricks): the padded quads and a tiled
         // TMA map over them
         const int nbx = (f.grid_n[0] + kSplineBrick - 1) / kSplineBrick, nby = (f.grid_n[1] + kSplineBrick - 1) / kSplineBrick,

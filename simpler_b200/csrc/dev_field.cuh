@@ -96,19 +96,10 @@ __device__ __forceinline__ void bessel_pair_clamped(const FieldParams &F, const 
     jm1 = fmaf(fmaf(fmaf(b.w, f, b.z), f, b.y), f, b.x);
 }
 
-// The same field in one straight line, for the march. A point off the axis and inside the table --
-// practically all of them -- needs no branch; the two tests that find the others are off the step's
-// dependency chain and share one branch at its end. (Each test as a branch of its own before the
-// lookup held the whole chain up until it resolved: the lone tail photon's step took 295 cycles.)
+// n and grad n at (y, z) off the axis from J_M and J_{M+1}, 1/r and A = n_max s
 template <int M>
-__device__ __forceinline__ void bessel_field_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
-    const float y = p.y, z = p.z;
-    const float r2 = fmaxf(fmaf(y, y, z * z), 1e-20f);       // a point below is rare anyway: r < kEps
-    const float rs = rsqrt_fast(r2);
-    const float A = F.amp * s;
-    const float r = r2 * rs, t = F.kb * r;
-    float jm, jm1;
-    bessel_pair_clamped(F, tab, t, jm, jm1);
+__device__ __forceinline__ void bessel_result(const FieldParams &F, float A, float y, float z, float rs, float jm, float jm1,
+                                              float &n, float3 &g) {
     if (M == 0) {
         // grad = A k J_0'(kr) (0, y, z)/r = -A k J_1(kr) (0, y, z)/r
         n = fmaf(A, jm, F.n_o);
@@ -130,6 +121,22 @@ __device__ __forceinline__ void bessel_field_ng(const FieldParams &F, const floa
         const float a2 = A * jm * float(M) * sm * rs * rs;
         g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
     }
+}
+
+// The same field in one straight line, for the march. A point off the axis and inside the table --
+// practically all of them -- needs no branch; the two tests that find the others are off the step's
+// dependency chain and share one branch at its end. (Each test as a branch of its own before the
+// lookup held the whole chain up until it resolved: the lone tail photon's step took 295 cycles.)
+template <int M>
+__device__ __forceinline__ void bessel_field_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+    const float y = p.y, z = p.z;
+    const float r2 = fmaxf(fmaf(y, y, z * z), 1e-20f);       // a point below is rare anyway: r < kEps
+    const float rs = rsqrt_fast(r2);
+    const float A = F.amp * s;
+    const float r = r2 * rs, t = F.kb * r;
+    float jm, jm1;
+    bessel_pair_clamped(F, tab, t, jm, jm1);
+    bessel_result<M>(F, A, y, z, rs, jm, jm1, n, g);
     if (!((r >= kEps) & (t < F.bend))) {
         const float4 q = bessel_field_rare<M>(F, tab, p, s);
         n = q.w;
@@ -234,9 +241,8 @@ __device__ __forceinline__ int spline_wrap(int i, int n) {
     if (w < 0) w += m;
     return w >= n ? m - w : w;
 }
-__device__ __forceinline__ void bspline_weights(float t, float w[4], float dw[4]) {
-    // taps at floor(t)-1 .. floor(t)+2, offsets d = t - i in (1,2], (0,1], (-1,0], (-2,-1]
-    float f = t - floorf(t);
+// f = t - floor(t): taps at floor(t)-1 .. floor(t)+2, offsets d = t - i in (1,2], (0,1], (-1,0], (-2,-1]
+__device__ __forceinline__ void bspline_weights_f(float f, float w[4], float dw[4]) {
     float f2 = f * f, f3v = f2 * f;
     float g = 1.0f - f;
     w[0] = g * g * g * (1.0f / 6.0f);
@@ -247,6 +253,16 @@ __device__ __forceinline__ void bspline_weights(float t, float w[4], float dw[4]
     dw[1] = (1.5f * f - 2.0f) * f;
     dw[2] = -(1.5f * g - 2.0f) * g;
     dw[3] = 0.5f * f2;
+}
+__device__ __forceinline__ void bspline_weights(float t, float w[4], float dw[4]) {
+    bspline_weights_f(t - floorf(t), w, dw);
+}
+// Cell and offset of a grid coordinate without conversions: a round-down add of 2^23 + 64 leaves
+// floor(t) + 64 in the low bits. A t outside [-64, 2^23) or not a number gives a cell far off any grid.
+__device__ __forceinline__ int spline_cell_of(float t, float &f) {
+    const float tb = __fadd_rd(t, 8388672.0f);
+    f = t - (tb - 8388672.0f);
+    return __float_as_int(tb) - (0x4B000000 + 64);
 }
 // The march kernel of the slot pool stages one brick of the coefficient grid in shared memory (the
 // x-tap quads of kSplineBrick^3 cells and their rows' one-cell apron below and two-cell apron above
@@ -286,24 +302,32 @@ __device__ __forceinline__ void spline_result(const FieldParams &F, const Spline
 // is a tenth of a cell or less on the usual grids (0.01 mm steps on 64 to 96 nodes over 10 mm), so
 // a march reads its taps once per cell instead of once per step.
 struct SplineCell {
-    int bx, by, bz;
+    int x, y, z;
     float4 q[16];
-    __device__ __forceinline__ void clear() { bx = by = bz = INT_MIN; }    // no cell starts there
+    __device__ __forceinline__ void clear() {                      // no cell
+        x = y = z = INT_MIN;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) q[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
 };
 
-// The rows of the cell whose taps start at (bx, by, bz), sixteen independent 16-byte loads.
-__device__ __forceinline__ void spline_rows(const FieldParams &F, int bx, int by, int bz, float4 q[16]) {
-    const int N0 = F.N[0], N1 = F.N[1], N2 = F.N[2];
+// The tap rows of cell (x, y, z), sixteen independent 16-byte loads: a cell of the grid or the one next
+// to it on any side (a step that overshoots a face is evaluated there before it is taken back).
+__device__ __forceinline__ bool spline_on_quads(const FieldParams &F, int x, int y, int z) {
+    return (F.coeff4 != nullptr) & (unsigned(x + 1) < unsigned(F.N[0] + 2)) & (unsigned(y + 1) < unsigned(F.N[1] + 2)) &
+           (unsigned(z + 1) < unsigned(F.N[2] + 2));
+}
+__device__ __forceinline__ void spline_rows(const FieldParams &F, int x, int y, int z, float4 q[16]) {
     int iy[4], iz[4];
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        iy[a] = spline_wrap(by + a, N1) * N0;
-        iz[a] = spline_wrap(bz + a, N2) * N0 * N1;
+        iy[a] = spline_wrap(y - 1 + a, F.N[1]) * F.qrow;
+        iz[a] = spline_wrap(z - 1 + a, F.N[2]) * F.N[1] * F.qrow;
     }
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) q[4 * c + b] = __ldg(F.coeff4 + (iz[c] + iy[b] + bx + 1));
+        for (int b = 0; b < 4; ++b) q[4 * c + b] = __ldg(F.coeff4 + (iz[c] + iy[b] + x));
 }
 
 // taps read one by one: a point off the grid in x, or a plan without quads. Returns (grad n, n).
@@ -332,32 +356,39 @@ static __device__ __noinline__ float4 spline_taps(const FieldParams &F, float3 p
 
 __device__ __forceinline__ bool spline_in_gap(const FieldParams &F, float3 p) { return p.x > F.egap || p.x < F.sgap; }
 
-// n and grad n with the taps of the march's current cell kept in C
+// n and grad n with the taps of the march's current cell kept in C. A straight line but for the reload:
+// a point off the grid is redone with the taps one by one at the end.
 __device__ __forceinline__ void spline_field_cell(const FieldParams &F, SplineCell &C, float3 p, float &n, float3 &g) {
-    const float tx = (p.x - F.xmin[0]) * F.xres[0], ty = (p.y - F.xmin[1]) * F.xres[1], tz = (p.z - F.xmin[2]) * F.xres[2];
-    const int bx = int(floorf(tx)) - 1, by = int(floorf(ty)) - 1, bz = int(floorf(tz)) - 1;
+    float fx, fy, fz;
+    const int x = spline_cell_of((p.x - F.xmin[0]) * F.xres[0], fx), y = spline_cell_of((p.y - F.xmin[1]) * F.xres[1], fy),
+              z = spline_cell_of((p.z - F.xmin[2]) * F.xres[2], fz);
+    const bool on = spline_on_quads(F, x, y, z);
+    // the lanes that reload meet the others again before the arithmetic: left alone they ran it apart
+    // (1.7 times the instructions)
+    const unsigned together = __activemask();
+    if (on & ((x != C.x) | (y != C.y) | (z != C.z))) {
+        spline_rows(F, x, y, z, C.q);
+        C.x = x; C.y = y; C.z = z;
+    }
+    __syncwarp(together);
     SplineW w;
-    spline_weights(tx, ty, tz, w);
+    bspline_weights_f(fx, w.wx, w.dx);
+    bspline_weights_f(fy, w.wy, w.dy);
+    bspline_weights_f(fz, w.wz, w.dz);
     SplineSum s = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (F.coeff4 != nullptr && unsigned(bx + 1) < unsigned(F.N[0])) {
-        if ((bx != C.bx) | (by != C.by) | (bz != C.bz)) {
-            spline_rows(F, bx, by, bz, C.q);
-            C.bx = bx; C.by = by; C.bz = bz;
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const float4 q = C.q[4 * c + b];
+            spline_row(w, b, c, q.x, q.y, q.z, q.w, s);
         }
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const float4 q = C.q[4 * c + b];
-                spline_row(w, b, c, q.x, q.y, q.z, q.w, s);
-            }
-    } else {
+    spline_result(F, s, n, g);
+    if (!on) {
         const float4 r = spline_taps(F, p);
         n = r.w;
         g = f3(r.x, r.y, r.z);
-        return;
     }
-    spline_result(F, s, n, g);
 }
 
 __device__ __forceinline__ void spline_field(const FieldParams &F, const float4 *brick, float3 p, float &n, float3 &g) {
@@ -392,9 +423,9 @@ __device__ __forceinline__ void spline_field(const FieldParams &F, const float4 
                 const float4 q = bq[(c * kSplineBrickRows + b) * kSplineBrick];
                 spline_row(w, b, c, q.x, q.y, q.z, q.w, s);
             }
-    } else if (F.coeff4 != nullptr && unsigned(bx + 1) < unsigned(F.N[0])) {
+    } else if (spline_on_quads(F, bx + 1, by + 1, bz + 1)) {
         float4 q[16];
-        spline_rows(F, bx, by, bz, q);
+        spline_rows(F, bx + 1, by + 1, bz + 1, q);
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
@@ -459,6 +490,18 @@ static __device__ __noinline__ float4 bessel_field_rt_rare(const FieldParams &F,
     bessel_field_rt_any(F, tab, p, s, n, g);
     return make_float4(g.x, g.y, g.z, n);
 }
+__device__ __forceinline__ void bessel_rt_result(const FieldParams &F, int M, float A, float y, float z, float rs, float jm,
+                                                 float jm1, float &n, float3 &g) {
+    const float c = z * rs, sn = y * rs;
+    const float cm = M == 0 ? 1.0f : (M == 1 ? c : fmaf(c, c, -sn * sn));
+    const float sm = M == 0 ? 0.0f : (M == 1 ? sn : 2.0f * c * sn);
+    n = fmaf(A * jm, cm, F.n_o);
+    const float fm = float(M);
+    const float djm = fmaf(fm * F.inv_k * rs, jm, -jm1);
+    const float a1 = A * djm * F.k_r * rs * cm;
+    const float a2 = A * jm * fm * sm * rs * rs;
+    g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
+}
 // in one straight line, as bessel_field_ng
 __device__ __forceinline__ void bessel_field_rt_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
     const int M = F.mode;
@@ -467,17 +510,9 @@ __device__ __forceinline__ void bessel_field_rt_ng(const FieldParams &F, const f
     const float r2 = fmaxf(fmaf(y, y, z * z), 1e-20f);
     const float rs = rsqrt_fast(r2);
     const float r = r2 * rs, t = F.kb * r;
-    const float c = z * rs, sn = y * rs;
-    const float cm = M == 0 ? 1.0f : (M == 1 ? c : fmaf(c, c, -sn * sn));
-    const float sm = M == 0 ? 0.0f : (M == 1 ? sn : 2.0f * c * sn);
     float jm, jm1;
     bessel_pair_clamped(F, tab, t, jm, jm1);
-    n = fmaf(A * jm, cm, F.n_o);
-    const float fm = float(M);
-    const float djm = fmaf(fm * F.inv_k * rs, jm, -jm1);
-    const float a1 = A * djm * F.k_r * rs * cm;
-    const float a2 = A * jm * fm * sm * rs * rs;
-    g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
+    bessel_rt_result(F, M, A, y, z, rs, jm, jm1, n, g);
     if (!((r >= kEps) & (t < F.bend))) {
         const float4 q = bessel_field_rt_rare(F, tab, p, s);
         n = q.w;
@@ -528,6 +563,82 @@ __device__ __forceinline__ void bessel_field_n_ng(const FieldParams &F, const fl
     const float a2 = A * jm * fm * sm * rs * rs;
     g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
 }
+// The whole warp on one spline photon. The sixteen tap rows of an evaluation are independent up to
+// their sums, which run in a fixed order. When a warp has one photon left, its 32 lanes march it
+// together (march.cuh spline_warp_march): every lane carries the whole march state and takes one
+// row's dot product (lanes 0-15 with the value weights, 16-31 with the derivative weights), the
+// products go through shared memory, and each of four lanes (all lanes, four by four) adds the
+// sixteen rows of one sum in spline_row's order. One lane alone issues about 470 instructions a step,
+// more than the instruction cache holds close, and took 535 ns.
+struct SplineWarp {
+    float s[2][16];            // row sums with the value (0) and derivative (1) weights
+    float w[3][16];            // their factors: wy wz, dy wz, wy dz
+};
+struct SplineWarpCell {
+    SplineWarp *buf;           // two, used in turn, so that one __syncwarp a step orders writes and reads
+    int turn, lane;
+    int x, y, z;
+    float4 r;                  // this lane's row
+};
+
+// weight and derivative weight of tap `a` alone: the expressions of bspline_weights_f with g for f where
+// that tap's are written in g (0.5 g g g is 0.5 (g g g): halving is exact)
+__device__ __forceinline__ void bspline_tap(float f, int a, float &w, float &dw) {
+    const bool low = (a & 1) == (a >> 1);             // taps 0 and 3: the outer ones
+    const bool neg = a == 0 || a == 2;                // in g = 1 - f
+    const float u = neg ? 1.0f - f : f;
+    const float u2 = u * u, u3 = u2 * u;
+    w = low ? u3 * (1.0f / 6.0f) : (2.0f / 3.0f) - u2 + 0.5f * u3;
+    const float d = low ? 0.5f * u2 : (1.5f * u - 2.0f) * u;
+    dw = neg ? -d : d;
+}
+
+// The evaluation above; every lane of the warp calls it with the same p.
+__device__ __forceinline__ void spline_field_cell(const FieldParams &F, SplineWarpCell &C, float3 p, float &n, float3 &g) {
+    float fx, fy, fz;
+    const int x = spline_cell_of((p.x - F.xmin[0]) * F.xres[0], fx), y = spline_cell_of((p.y - F.xmin[1]) * F.xres[1], fy),
+              z = spline_cell_of((p.z - F.xmin[2]) * F.xres[2], fz);
+    if (spline_on_quads(F, x, y, z)) {
+        const int row = C.lane & 15, b = row & 3, c = row >> 2, half = C.lane >> 4, q = C.lane & 3;
+        if ((x != C.x) | (y != C.y) | (z != C.z)) {
+            C.r = __ldg(F.coeff4 + ((spline_wrap(z - 1 + c, F.N[2]) * F.N[1] + spline_wrap(y - 1 + b, F.N[1])) * F.qrow + x));
+            C.x = x; C.y = y; C.z = z;
+        }
+        SplineWarp &B = C.buf[C.turn];
+        C.turn ^= 1;
+        float wy, dy, wz, dz, wx[4], dx[4];
+        bspline_tap(fy, b, wy, dy);
+        bspline_tap(fz, c, wz, dz);
+        bspline_weights_f(fx, wx, dx);
+        B.w[half ? 2 : 0][row] = wy * (half ? dz : wz);
+        B.w[1][row] = dy * wz;
+        if (half) { wx[0] = dx[0]; wx[1] = dx[1]; wx[2] = dx[2]; wx[3] = dx[3]; }
+        B.s[half][row] = C.r.x * wx[0] + C.r.y * wx[1] + C.r.z * wx[2] + C.r.w * wx[3];
+        __syncwarp();
+        const float4 *sp = reinterpret_cast<const float4 *>(B.s[q == 1 ? 1 : 0]);
+        const float4 *wp = reinterpret_cast<const float4 *>(B.w[q < 2 ? 0 : q - 1]);
+        float sum = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float4 u = sp[e], v = wp[e];
+            sum = fmaf(u.x, v.x, sum);
+            sum = fmaf(u.y, v.y, sum);
+            sum = fmaf(u.z, v.z, sum);
+            sum = fmaf(u.w, v.w, sum);
+        }
+        SplineSum T;
+        T.v = __shfl_sync(0xffffffffu, sum, 0);
+        T.gx = __shfl_sync(0xffffffffu, sum, 1);
+        T.gy = __shfl_sync(0xffffffffu, sum, 2);
+        T.gz = __shfl_sync(0xffffffffu, sum, 3);
+        spline_result(F, T, n, g);
+    } else {
+        const float4 e = spline_taps(F, p);
+        n = e.w;
+        g = f3(e.x, e.y, e.z);
+    }
+}
+
 // Field<FK>: the field of one kind. tab is the Bessel table (shared memory in the march kernel) or
 // the staged spline brick, unused by the other kinds.
 //   eval(F, tab, p, s, n, g)          n and grad n at p
@@ -572,7 +683,9 @@ template <> struct Field<FK_SPLINE> {
         spline_field(F, nullptr, p, n, g);
         return make_float4(g.x, g.y, g.z, n);
     }
-    static __device__ __forceinline__ void eval_c(const FieldParams &F, const float4 *, Cache &C, float3 p, float, float &n, float3 &g) {
+    // CA: a SplineCell, or the whole warp's cell (SplineWarpCell)
+    template <class CA>
+    static __device__ __forceinline__ void eval_c(const FieldParams &F, const float4 *, CA &C, float3 p, float, float &n, float3 &g) {
         if (spline_in_gap(F, p)) {
             n = F.n_o;
             g = f3(0.0f, 0.0f, 0.0f);
@@ -580,7 +693,8 @@ template <> struct Field<FK_SPLINE> {
         }
         spline_field_cell(F, C, p, n, g);
     }
-    static __device__ __forceinline__ void eval_in(const FieldParams &F, const float4 *, Cache &C, float3 p, float, float &n, float3 &g) {
+    template <class CA>
+    static __device__ __forceinline__ void eval_in(const FieldParams &F, const float4 *, CA &C, float3 p, float, float &n, float3 &g) {
         spline_field_cell(F, C, p, n, g);
     }
 };

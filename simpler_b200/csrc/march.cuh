@@ -484,30 +484,186 @@ __device__ __forceinline__ int safe_steps(const S &L, const KParams &P, int cap)
     return min(int(fminf(k, float(cap))), L.stop - L.steps - 1);
 }
 
-// `k` steps of march_step that safe_steps has shown to be accepted
-template <int FK, class S>
-__device__ __forceinline__ void march_window(S &L, const KParams &P, int k, typename Field<FK>::Cache &C) {
+// The field along a window. begin(p, v, h/n) starts (or restarts) it at a point, eval(p) gives n and
+// grad n at the next point and false where it could not (the caller then takes the field from
+// Field<FK>::eval_in). The same bits either way.
+template <int FK, class CA> struct WindowField {
+    CA &C;
+    const FieldParams &F;
+    const float4 *tab;
+    float s;
+    __device__ __forceinline__ void begin(float3, float3, float) {}
+    __device__ __forceinline__ bool eval(float3 p, float &n, float3 &g) {
+        Field<FK>::eval_in(F, tab, C, p, s, n, g);
+        return true;
+    }
+};
+// Bessel modes 0-2 (RT: by the batched sweep's order-general formulas). The table entry a step needs
+// is known one step ahead all but always: the table coordinate t moves by nearly the same amount
+// each step. So the entry of the interval t + dt falls in is loaded while the step before it is still
+// under way, which takes the index, the address and the load off the chain of dependent
+// instructions; a point in another interval (or off the table, or on the axis) fails f's test.
+template <int M, bool RT> struct WindowBessel {
+    const FieldParams &F;
+    const float4 *tab;
+    float s;
+    float t, fi;
+    float4 a, b;
+    __device__ __forceinline__ void load(float tp) {
+        const float big = 8388608.0f;
+        const float tb = fminf(__fadd_rd(fmaxf(tp, 0.0f), big), big + (F.bend - 1.0f));
+        const unsigned i = unsigned(__float_as_int(tb) - 0x4B000000);
+        fi = tb - big;
+        a = tab[2 * i];
+        b = tab[2 * i + 1];
+    }
+    __device__ __forceinline__ void begin(float3 p, float3 v, float hinv) {
+        const float r2 = fmaf(p.y, p.y, p.z * p.z), rs = rsqrt_fast(r2);
+        t = F.kb * (r2 * rs);
+        load(fmaf(F.kb * rs * hinv, fmaf(p.y, v.y, p.z * v.z), t));
+    }
+    __device__ __forceinline__ bool eval(float3 p, float &n, float3 &g) {
+        const float y = p.y, z = p.z;
+        const float r2 = fmaf(y, y, z * z);
+        const float rs = rsqrt_fast(r2);
+        const float r = r2 * rs, tn = F.kb * r;
+        const float f = tn - fi;
+        const bool ok = (r >= kEps) & (f >= 0.0f) & (f < 1.0f);
+        const float jm = fmaf(fmaf(fmaf(a.w, f, a.z), f, a.y), f, a.x);
+        const float jm1 = fmaf(fmaf(fmaf(b.w, f, b.z), f, b.y), f, b.x);
+        load(tn + (tn - t));
+        t = tn;
+        if (RT) bessel_rt_result(F, M, F.amp * s, y, z, rs, jm, jm1, n, g);
+        else bessel_result<M>(F, F.amp * s, y, z, rs, jm, jm1, n, g);
+        return ok;
+    }
+};
+
+// `k` steps of march_step (a multiple of four) that safe_steps has shown to be accepted, in blocks of
+// four without a branch (one for the spline, whose unrolled step does not fit the instruction cache
+// four times: 633 against 535 ns a step); a block in which the field's prediction failed runs again
+// from its start.
+template <int FK, int FP, class S, class CA, class WF>
+__device__ __forceinline__ void window_steps(S &L, const KParams &P, int k, CA &C, WF W) {
     const FieldParams &F = field_of<FK>(L, P);
     const float h = L.cur, hh = L.hh, s = L.s;
     const double hd = L.cur_d;
-    const bool f64 = P.fp64 != 0;
     float3 p = L.mp, v = L.md, g = L.mg;
     float n = L.mn, acc = L.dist_acc, totf = L.mtotf;
     double tot = L.mtot;
+    W.begin(p, v, h * rcp_fast(n));
+    constexpr int B = FK == FK_SPLINE ? 1 : 4;
 #pragma unroll 1
-    for (int i = 0; i < k; ++i) {
-        const float3 d = f3(fmaf(hh, g.x, v.x), fmaf(hh, g.y, v.y), fmaf(hh, g.z, v.z));
-        const float hinv = h * rcp_fast(n);
-        p = f3(fmaf(d.x, hinv, p.x), fmaf(d.y, hinv, p.y), fmaf(d.z, hinv, p.z));
-        Field<FK>::eval_in(F, L.tab, C, p, s, n, g);
-        v = f3(fmaf(hh, g.x, d.x), fmaf(hh, g.y, d.y), fmaf(hh, g.z, d.z));
-        acc = acc + h;
-        if (f64) tot = fma(hd, double(n), tot);
-        else totf = fmaf(h, n, totf);
+    for (int i = 0; i < k; i += B) {
+        const float3 p0 = p, v0 = v, g0 = g;
+        const float n0 = n, acc0 = acc, totf0 = totf;
+        const double tot0 = tot;
+        bool ok = true;
+#pragma unroll
+        for (int j = 0; j < B; ++j) {
+            const float3 d = f3(fmaf(hh, g.x, v.x), fmaf(hh, g.y, v.y), fmaf(hh, g.z, v.z));
+            const float hinv = h * rcp_fast(n);
+            p = f3(fmaf(d.x, hinv, p.x), fmaf(d.y, hinv, p.y), fmaf(d.z, hinv, p.z));
+            ok &= W.eval(p, n, g);
+            v = f3(fmaf(hh, g.x, d.x), fmaf(hh, g.y, d.y), fmaf(hh, g.z, d.z));
+            acc = acc + h;
+            if (FP) tot = fma(hd, double(n), tot);
+            else totf = fmaf(h, n, totf);
+        }
+        if (!ok) {
+            p = p0; v = v0; g = g0; n = n0; acc = acc0; totf = totf0; tot = tot0;
+#pragma unroll 1
+            for (int j = 0; j < B; ++j) {
+                const float3 d = f3(fmaf(hh, g.x, v.x), fmaf(hh, g.y, v.y), fmaf(hh, g.z, v.z));
+                const float hinv = h * rcp_fast(n);
+                p = f3(fmaf(d.x, hinv, p.x), fmaf(d.y, hinv, p.y), fmaf(d.z, hinv, p.z));
+                Field<FK>::eval_in(F, L.tab, C, p, s, n, g);
+                v = f3(fmaf(hh, g.x, d.x), fmaf(hh, g.y, d.y), fmaf(hh, g.z, d.z));
+                acc = acc + h;
+                if (FP) tot = fma(hd, double(n), tot);
+                else totf = fmaf(h, n, totf);
+            }
+            W.begin(p, v, h * rcp_fast(n));
+        }
     }
     L.mp = p; L.md = v; L.mg = g; L.mn = n;
     L.dist_acc = acc; L.mtotf = totf; L.mtot = tot;
     L.steps += k;
+}
+
+template <int FK, int FP, class S, class CA>
+__device__ __forceinline__ void march_window_fp(S &L, const KParams &P, int k, CA &C) {
+    const FieldParams &F = field_of<FK>(L, P);
+    if constexpr (FK <= FK_BESSEL2) {
+        window_steps<FK, FP>(L, P, k, C, WindowBessel<FK, false>{F, L.tab, L.s});
+    } else if constexpr (FK == FK_BATCH) {
+        if (F.mode == 0) window_steps<FK, FP>(L, P, k, C, WindowBessel<0, true>{F, L.tab, L.s});
+        else if (F.mode == 1) window_steps<FK, FP>(L, P, k, C, WindowBessel<1, true>{F, L.tab, L.s});
+        else window_steps<FK, FP>(L, P, k, C, WindowBessel<2, true>{F, L.tab, L.s});
+    } else {
+        window_steps<FK, FP>(L, P, k, C, WindowField<FK, CA>{C, F, L.tab, L.s});
+    }
+}
+template <int FK, class S, class CA>
+__device__ __forceinline__ void march_window(S &L, const KParams &P, int k, CA &C) {
+    if (P.fp64) march_window_fp<FK, 1>(L, P, k, C);
+    else march_window_fp<FK, 0>(L, P, k, C);
+}
+
+// ---- a lone spline photon on the whole warp ------------------------------------------------------
+// Marches the photon of lane `src`, the warp's last, to the end of its march with the whole warp
+// (SplineWarpCell): the lane's march state in every lane, the same windows and steps in all of them,
+// the result back to the owner. Returns the accepted steps. All 32 lanes call it.
+__device__ __forceinline__ int spline_warp_march(Lane &L, const KParams &P, int src, SplineWarp *buf, int lane) {
+    struct {
+        float3 mp, md, mg;
+        float mn, cur, hh, dist_acc, dlimit, mtotf, s;
+        double mtot, cur_d;
+        int steps, stop, prec, end;
+        const float4 *tab;
+        const Inst *inst;
+    } M;
+    auto from = [&](float x) { return __shfl_sync(kFull, x, src); };
+    auto fromi = [&](int x) { return __shfl_sync(kFull, x, src); };
+    M.mp = f3(from(L.mp.x), from(L.mp.y), from(L.mp.z));
+    M.md = f3(from(L.md.x), from(L.md.y), from(L.md.z));
+    M.mg = f3(from(L.mg.x), from(L.mg.y), from(L.mg.z));
+    M.mn = from(L.mn); M.cur = from(L.cur); M.hh = from(L.hh);
+    M.dist_acc = from(L.dist_acc); M.dlimit = from(L.dlimit); M.mtotf = from(L.mtotf);
+    M.mtot = __shfl_sync(kFull, L.mtot, src);
+    M.cur_d = __shfl_sync(kFull, L.cur_d, src);
+    M.steps = fromi(L.steps); M.stop = fromi(L.stop); M.prec = fromi(L.prec); M.end = fromi(L.end);
+    M.s = 0.0f;
+    M.tab = nullptr;
+    M.inst = nullptr;
+    SplineWarpCell C;
+    C.buf = buf; C.turn = 0; C.lane = lane;
+    C.x = C.y = C.z = INT_MIN;
+    C.r = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    __syncwarp();
+    int accepted = 0;
+    for (bool end = false; !end;) {
+        const int w = safe_steps<FK_SPLINE>(M, P, 1024);
+        if (w >= 4) {
+            march_window<FK_SPLINE>(M, P, w, C);
+            accepted += w;
+            continue;
+        }
+#pragma unroll 1
+        for (int t = 0; t < 8 && !end; ++t) {
+            const float3 q = M.mp;
+            end = march_step<FK_SPLINE>(M, P, C);
+            accepted += (q.x != M.mp.x || q.y != M.mp.y || q.z != M.mp.z) ? 1 : 0;
+        }
+    }
+    __syncwarp();
+    if (lane == src) {
+        L.mp = M.mp; L.md = M.md; L.mg = M.mg; L.mn = M.mn;
+        L.cur = M.cur; L.hh = M.hh; L.cur_d = M.cur_d;
+        L.dist_acc = M.dist_acc; L.mtotf = M.mtotf; L.mtot = M.mtot;
+        L.steps = M.steps; L.stop = M.stop; L.prec = M.prec; L.end = M.end;
+    }
+    return accepted;
 }
 
 // ---- discrete logic between marches ---------------------------------------------------------
@@ -833,6 +989,7 @@ static __device__ __noinline__ bool stage_to_shared(void *dst, const void *src, 
 // kernels use NoHook.
 template <int FK, class H = NoHook>
 __device__ __forceinline__ void lane_loop(Lane &L, int st, const KParams &P, LaneStats &S, int lane, H *h = nullptr) {
+    __shared__ __align__(16) SplineWarp s_warp[FK == FK_SPLINE ? 8 : 1];      // 128-thread blocks
     int pending_ev = EV_NEW;
     for (;;) {
         for (;;) {
@@ -874,12 +1031,23 @@ __device__ __forceinline__ void lane_loop(Lane &L, int st, const KParams &P, Lan
         typename Field<FK>::Cache C;
         C.clear();
         for (;;) {
+            if constexpr (FK == FK_SPLINE) {
+                if ((alive & (alive - 1u)) == 0u) {
+                    const int n = spline_warp_march(L, P, __ffs(alive) - 1, s_warp + 2 * (threadIdx.x >> 5), lane);
+                    if (st == ST_MARCH) {
+                        if (H::on) h->accepted(n);
+                        st = ST_EVENT;
+                        pending_ev = EV_MARCH_END;
+                    }
+                    break;
+                }
+            }
             if (st == ST_MARCH) {
                 bool end = false;
                 const int w = FK == FK_SOURCES ? 0 : safe_steps<FK>(L, P, wcap);
                 if (w >= 4) {
-                    march_window<FK>(L, P, w, C);
-                    if (H::on) h->accepted(w);
+                    march_window<FK>(L, P, w & ~3, C);
+                    if (H::on) h->accepted(w & ~3);
                 } else {
 #pragma unroll 1
                     for (int t = 0; t < (FK == FK_SOURCES ? 2 : 8) && !end; ++t) {
