@@ -363,14 +363,10 @@ __device__ __forceinline__ void spline_field_cell(const FieldParams &F, SplineCe
     const int x = spline_cell_of((p.x - F.xmin[0]) * F.xres[0], fx), y = spline_cell_of((p.y - F.xmin[1]) * F.xres[1], fy),
               z = spline_cell_of((p.z - F.xmin[2]) * F.xres[2], fz);
     const bool on = spline_on_quads(F, x, y, z);
-    // the lanes that reload meet the others again before the arithmetic: left alone they ran it apart
-    // (1.7 times the instructions)
-    const unsigned together = __activemask();
     if (on & ((x != C.x) | (y != C.y) | (z != C.z))) {
         spline_rows(F, x, y, z, C.q);
         C.x = x; C.y = y; C.z = z;
     }
-    __syncwarp(together);
     SplineW w;
     bspline_weights_f(fx, w.wx, w.dx);
     bspline_weights_f(fy, w.wy, w.dy);

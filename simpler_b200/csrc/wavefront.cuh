@@ -262,11 +262,9 @@ wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveP
         const bool valid = i < n;
         bool ended = false;
         int slot = 0;
-        MarchState M;
-        float inst_bits = 0.0f;
-        int steps0 = 0;
         if (valid) {
             slot = two_class_at(W.list[cur], n0, W.n_slots, i);
+            MarchState M;
             const float4 a = W.ma[slot], b = W.mb[slot], c = W.mc[slot], d = W.mdd[slot];
             const int4 e = W.mi[slot];
             M.mp = f3(a.x, a.y, a.z); M.mn = a.w;
@@ -277,37 +275,30 @@ wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveP
             M.hh = 0.5f * M.cur;
             M.cur_d = double(M.cur);
             M.mtot = F64 ? W.mt[slot] : 0.0;
-            inst_bits = d.w;
             if (FK == FK_BATCH) {
                 M.inst = P.insts + __float_as_int(d.w);
                 M.tab = M.inst->field.btab;
             } else {
                 M.tab = FK == FK_SPLINE ? nullptr : smem_tab;   // no staged brick: global quads
             }
-            steps0 = M.steps;
-        }
-        typename Field<FK>::Cache C;
-        C.clear();
-        if (FK == FK_SPLINE) {
-            // one step a turn (the body of two does not fit the instruction cache), all lanes together
-            // at its end
+            const int steps0 = M.steps;
+            typename Field<FK>::Cache C;
+            C.clear();
+            if (FK == FK_SPLINE) {
+                // one step a turn: the body of two does not fit the instruction cache
 #pragma unroll 1
-            for (int k = 0; k < chunk; ++k) {
-                if (valid && !ended) ended = march_step<FK, F64>(M, P, C);
-                if (!__any_sync(kFull, valid && !ended)) break;
+                for (int k = 0; k < chunk && !ended; ++k) ended = march_step<FK, F64>(M, P, C);
+            } else {
+                for (int k = 0; k < chunk; k += 2) {
+                    if (march_step<FK, F64>(M, P, C) || march_step<FK, F64>(M, P, C)) { ended = true; break; }
+                }
             }
-        } else if (valid) {
-            for (int k = 0; k < chunk; k += 2) {
-                if (march_step<FK, F64>(M, P, C) || march_step<FK, F64>(M, P, C)) { ended = true; break; }
-            }
-        }
-        if (valid) {
             done += unsigned(M.steps - steps0);
             W.ma[slot] = make_float4(M.mp.x, M.mp.y, M.mp.z, M.mn);
             W.mb[slot] = make_float4(M.md.x, M.md.y, M.md.z, M.cur);
             W.mc[slot] = make_float4(M.mg.x, M.mg.y, M.mg.z, M.dist_acc);
             if (F64) W.mt[slot] = M.mtot;
-            else W.mdd[slot] = make_float4(M.dlimit, M.s, M.mtotf, inst_bits);
+            else W.mdd[slot] = make_float4(M.dlimit, M.s, M.mtotf, d.w);
             W.mi[slot] = make_int4(M.steps, M.end, M.prec, M.stop);
         }
         const unsigned em = __ballot_sync(kFull, valid && ended);
