@@ -523,6 +523,8 @@ struct smp_plan {
     int wave_chunk = 96;
     int wave_slots_per_lane = 6;
     int march_block = 128;      // threads per march-kernel block (128 or 256)
+    bool block_fixed = false;   // SMP_WF_BLOCK
+    int march_copies = 1;       // copies of the Bessel table in the march kernel's shared memory
     bool tuned = false;         // the schedule came from smp_plan_tune
     size_t wave_cap = 0;        // slots the pool allocation holds
     long long direct_max = 40000;   // renders of at most this many photons are one launch of the tail
@@ -758,7 +760,10 @@ int smp_plan_create(const smp_scene_desc *scene, const smp_medium_desc *medium, 
     if (const char *c = std::getenv("SMP_WF_TUNE")) p->tune_chunk = p->tune_chunk && std::atoi(c) != 0;
     if (const char *c = std::getenv("SMP_WF_GRAPH")) p->use_graph = std::atoi(c) != 0;
     if (const char *c = std::getenv("SMP_WF_SLOTS")) p->wave_slots_per_lane = std::max(1, std::min(16, std::atoi(c)));
-    if (const char *c = std::getenv("SMP_WF_BLOCK")) p->march_block = std::atoi(c) == 256 ? 256 : 128;
+    if (const char *c = std::getenv("SMP_WF_BLOCK")) {
+        p->march_block = std::atoi(c) == 256 ? 256 : 128;
+        p->block_fixed = true;
+    }
     if (const char *c = std::getenv("SMP_WF_BATCH")) p->wave_batch = std::max(1, std::min(256, std::atoi(c)));
     if (const char *c = std::getenv("SMP_WF_DIRECT")) p->direct_max = std::atoll(c);
     if (const char *c = std::getenv("SMP_WF_FINISH")) p->finish_max = std::atoll(c);
@@ -918,9 +923,18 @@ static int finish_setup(smp_plan *p) {
 
 static int wave_setup(smp_plan *p) {
     const bool bricks = p->fk == FK_SPLINE && p->bricks;
-    WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, bricks), fe = wf_event_fn(p->fk);
+    // copies of the Bessel table (dev_field.cuh RepTable) as long as the SM's resident blocks hold them:
+    // four in blocks of 256 up to k r = 36, two up to k r = 73, of which an untuned plan takes the first
+    // (5e6 photons of the precision scale-up: march kernel 273 ms with one copy, 264 with two in blocks
+    // of 128, 254 with four in blocks of 256)
+    auto fits = [p](int block) {
+        return p->fk <= FK_BESSELN && (p->smem_bytes * march_copies(block) + 1024) * size_t(6 * 128 / block) <= 220 * 1024;
+    };
+    if (!p->tuned && !p->block_fixed) p->march_block = fits(256) ? 256 : 128;
+    p->march_copies = fits(p->march_block) ? march_copies(p->march_block) : 1;
+    WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, bricks, p->march_copies), fe = wf_event_fn(p->fk);
     if (!fm || !fe) return set_error(SMP_ERR_BAD_ARG, "bad field kind");
-    p->march_smem = bricks ? size_t(kBrickSmemBytes) : p->smem_bytes;
+    p->march_smem = bricks ? size_t(kBrickSmemBytes) : p->smem_bytes * size_t(p->march_copies);
     int sms = 0, pm = 0, pe = 0;
     int rc = allow_dynamic_smem(reinterpret_cast<const void *>(fm), p->march_smem);
     if (!rc) rc = finish_setup(p);
@@ -1033,7 +1047,7 @@ static int wave_run(smp_plan *p, const KParams &k, cudaStream_t s) {
     }
     int rc = wave_setup(p);
     if (rc) return rc;
-    WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, p->wp.nb > 0), fe = wf_event_fn(p->fk),
+    WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, p->wp.nb > 0, p->march_copies), fe = wf_event_fn(p->fk),
            ff = wf_finish_fn(p->fk);
     WaveParams W = p->wp;
     const int mb = p->march_block;
@@ -2189,11 +2203,11 @@ static cudaError_t adjoint_trace_pool(smp_plan *p, const KParams &k, const AdjPa
                                       int grid_f, long long *launches) {
     WaveParams W = p->wp;
     W.nb = 0;
-    WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, false);
+    WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, false, p->march_copies);
     if (!fm) return cudaErrorInvalidDeviceFunction;
-    if (p->smem_bytes > 48 * 1024) {
+    if (p->march_smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void *>(fm), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(p->smem_bytes));
+                                             int(p->march_smem));
         if (e != cudaSuccess) return e;
     }
     const unsigned finish_at = unsigned(grid_f) * unsigned(kBlock);
@@ -2207,7 +2221,7 @@ static cudaError_t adjoint_trace_pool(smp_plan *p, const KParams &k, const AdjPa
     int par = 0;
     for (;;) {
         for (int j = 0; j < p->wave_batch; ++j, ++it) {
-            fm<<<p->grid_march, p->march_block, p->smem_bytes>>>(k, W, int(it & 0x3fffffff));
+            fm<<<p->grid_march, p->march_block, p->march_smem>>>(k, W, int(it & 0x3fffffff));
             fe<<<p->grid_event, kBlock>>>(k, W, a, int(it & 0x3fffffff));
         }
         *launches += 2 * p->wave_batch;

@@ -85,13 +85,36 @@ static __device__ __noinline__ float4 bessel_field_rare(const FieldParams &F, co
     return make_float4(g.x, g.y, g.z, n);
 }
 
+// The Bessel table as the march reads it. A plain pointer: entry i is tab[2i], tab[2i + 1]. RepTable<R>:
+// R copies of every 16-byte half side by side in shared memory, lane l reading copy l mod R. The lanes
+// of a warp look up unrelated radii, so the plain table's 16-byte loads collide in banks (the eight lanes
+// a wavefront serves share four 16-byte groups: about 14 wavefronts a load, and the L1/shared-memory
+// path at 86 % of its peak bounded the march kernel). With four copies two of the eight lanes share a
+// group: eight wavefronts.
+template <int R> struct RepTable {
+    const float4 *p;           // this lane's copy of entry 0
+};
+__device__ __forceinline__ void tab_load(const float4 *tab, unsigned i, float4 &a, float4 &b) {
+    a = tab[2 * i];
+    b = tab[2 * i + 1];
+}
+template <int R> __device__ __forceinline__ void tab_load(const RepTable<R> &tab, unsigned i, float4 &a, float4 &b) {
+    a = tab.p[2 * R * i];
+    b = tab.p[2 * R * i + R];
+}
+// the plain table, for the rare paths
+__device__ __forceinline__ const float4 *tab_plain(const FieldParams &, const float4 *tab) { return tab; }
+template <int R> __device__ __forceinline__ const float4 *tab_plain(const FieldParams &F, const RepTable<R> &) { return F.btab; }
+
 // (J_M, J_{M+1}) from the table at the coordinate t = k r / h, with no test on the way: the interval is
 // clamped to the table, and the caller redoes a point whose t is not below bend (or not a number).
-__device__ __forceinline__ void bessel_pair_clamped(const FieldParams &F, const float4 *tab, float t, float &jm, float &jm1) {
+template <class TAB>
+__device__ __forceinline__ void bessel_pair_clamped(const FieldParams &F, const TAB &tab, float t, float &jm, float &jm1) {
     const float tb = __fadd_rd(t, 8388608.0f);
     const unsigned i = min(unsigned(__float_as_int(tb) - 0x4B000000), unsigned(F.bint - 1));
     const float f = t - (tb - 8388608.0f);
-    const float4 a = tab[2 * i], b = tab[2 * i + 1];
+    float4 a, b;
+    tab_load(tab, i, a, b);
     jm = fmaf(fmaf(fmaf(a.w, f, a.z), f, a.y), f, a.x);
     jm1 = fmaf(fmaf(fmaf(b.w, f, b.z), f, b.y), f, b.x);
 }
@@ -127,8 +150,8 @@ __device__ __forceinline__ void bessel_result(const FieldParams &F, float A, flo
 // practically all of them -- needs no branch; the two tests that find the others are off the step's
 // dependency chain and share one branch at its end. (Each test as a branch of its own before the
 // lookup held the whole chain up until it resolved: the lone tail photon's step took 295 cycles.)
-template <int M>
-__device__ __forceinline__ void bessel_field_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+template <int M, class TAB>
+__device__ __forceinline__ void bessel_field_ng(const FieldParams &F, const TAB &tab, float3 p, float s, float &n, float3 &g) {
     const float y = p.y, z = p.z;
     const float r2 = fmaxf(fmaf(y, y, z * z), 1e-20f);       // a point below is rare anyway: r < kEps
     const float rs = rsqrt_fast(r2);
@@ -138,7 +161,7 @@ __device__ __forceinline__ void bessel_field_ng(const FieldParams &F, const floa
     bessel_pair_clamped(F, tab, t, jm, jm1);
     bessel_result<M>(F, A, y, z, rs, jm, jm1, n, g);
     if (!((r >= kEps) & (t < F.bend))) {
-        const float4 q = bessel_field_rare<M>(F, tab, p, s);
+        const float4 q = bessel_field_rare<M>(F, tab_plain(F, tab), p, s);
         n = q.w;
         g = f3(q.x, q.y, q.z);
     }
@@ -149,8 +172,8 @@ __device__ __forceinline__ bool in_gap(const FieldParams &F, float3 p) { return 
 
 // In the gaps the amplitude is zeroed instead of branching: n = n_o + 0 and grad n = 0 exactly,
 // and every lane runs the same instructions.
-template <int M>
-__device__ __forceinline__ void bessel_field(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+template <int M, class TAB>
+__device__ __forceinline__ void bessel_field(const FieldParams &F, const TAB &tab, float3 p, float s, float &n, float3 &g) {
     bessel_field_ng<M>(F, tab, p, in_gap(F, p) ? 0.0f : s, n, g);
 }
 
@@ -499,7 +522,8 @@ __device__ __forceinline__ void bessel_rt_result(const FieldParams &F, int M, fl
     g = f3(0.0f, fmaf(a1, y, -a2 * z), fmaf(a1, z, a2 * y));
 }
 // in one straight line, as bessel_field_ng
-__device__ __forceinline__ void bessel_field_rt_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+template <class TAB>
+__device__ __forceinline__ void bessel_field_rt_ng(const FieldParams &F, const TAB &tab, float3 p, float s, float &n, float3 &g) {
     const int M = F.mode;
     const float A = F.amp * s;
     const float y = p.y, z = p.z;
@@ -510,7 +534,7 @@ __device__ __forceinline__ void bessel_field_rt_ng(const FieldParams &F, const f
     bessel_pair_clamped(F, tab, t, jm, jm1);
     bessel_rt_result(F, M, A, y, z, rs, jm, jm1, n, g);
     if (!((r >= kEps) & (t < F.bend))) {
-        const float4 q = bessel_field_rt_rare(F, tab, p, s);
+        const float4 q = bessel_field_rt_rare(F, tab_plain(F, tab), p, s);
         n = q.w;
         g = f3(q.x, q.y, q.z);
     }
@@ -520,7 +544,8 @@ __device__ __forceinline__ void bessel_field_rt_ng(const FieldParams &F, const f
 // from the per-plan table, which the host sizes to cover the whole box (k r <= 128, checked when the
 // plan is made; a point beyond it reads the table's last interval); cos(m phi), sin(m phi) as
 // ((z + i y)/r)^m by m - 1 complex products.
-__device__ __forceinline__ void bessel_field_n_ng(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) {
+template <class TAB>
+__device__ __forceinline__ void bessel_field_n_ng(const FieldParams &F, const TAB &tab, float3 p, float s, float &n, float3 &g) {
     const int M = F.mode;
     const float A = F.amp * s;
     float y = p.y, z = p.z;
@@ -542,7 +567,8 @@ __device__ __forceinline__ void bessel_field_n_ng(const FieldParams &F, const fl
         const float tb = __fadd_rd(t, 8388608.0f);
         const int i = __float_as_int(tb) - 0x4B000000;
         const float f = t - (tb - 8388608.0f);
-        const float4 a = tab[2 * i], b = tab[2 * i + 1];
+        float4 a, b;
+        tab_load(tab, unsigned(i), a, b);
         jm = fmaf(fmaf(fmaf(a.w, f, a.z), f, a.y), f, a.x);
         jm1 = fmaf(fmaf(fmaf(b.w, f, b.z), f, b.y), f, b.x);
     };
@@ -648,9 +674,9 @@ template <int FK> struct Field;
 #define SMP_FIELD(FK, IN, ALL)                                                                                      \
     template <> struct Field<FK> {                                                                                  \
         using Cache = NoCache;                                                                                      \
-        static __device__ __forceinline__ void eval(const FieldParams &F, const float4 *tab, float3 p, float s, float &n, float3 &g) { ALL; } \
-        static __device__ __forceinline__ void eval_c(const FieldParams &F, const float4 *tab, Cache &, float3 p, float s, float &n, float3 &g) { ALL; } \
-        static __device__ __forceinline__ void eval_in(const FieldParams &F, const float4 *tab, Cache &, float3 p, float s, float &n, float3 &g) { IN; } \
+        template <class TAB> static __device__ __forceinline__ void eval(const FieldParams &F, const TAB &tab, float3 p, float s, float &n, float3 &g) { ALL; } \
+        template <class TAB> static __device__ __forceinline__ void eval_c(const FieldParams &F, const TAB &tab, Cache &, float3 p, float s, float &n, float3 &g) { ALL; } \
+        template <class TAB> static __device__ __forceinline__ void eval_in(const FieldParams &F, const TAB &tab, Cache &, float3 p, float s, float &n, float3 &g) { IN; } \
     };
 SMP_FIELD(FK_BESSEL0, bessel_field_ng<0>(F, tab, p, s, n, g), bessel_field<0>(F, tab, p, s, n, g))
 SMP_FIELD(FK_BESSEL1, bessel_field_ng<1>(F, tab, p, s, n, g), bessel_field<1>(F, tab, p, s, n, g))

@@ -73,7 +73,9 @@ __device__ __forceinline__ void sincos_red(float t, float &s, float &c) {
     const float kInv2Pi = 0.159154943091895335768f;
     const float k2PiHi = 6.28318548202514648438f;     // float(2*pi)
     const float k2PiLo = -1.74845553146951609e-07f;   // 2*pi - float(2*pi)
-    float q = rintf(t * kInv2Pi);
+    // rintf by an add that rounds to an integer (two adds instead of a conversion-pipe instruction, which
+    // shares its pipe with the sine and cosine)
+    float q = (t * kInv2Pi + 12582912.0f) - 12582912.0f;
     float r = fmaf(-q, k2PiHi, t);
     r = fmaf(-q, k2PiLo, r);
     __sincosf(r, &s, &c);

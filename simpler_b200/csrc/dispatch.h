@@ -24,7 +24,9 @@ MarchFn plain_fn(int fk);                        // one thread per photon (plain
 ProbeFn field_probe_fn(int fk);                  // field at host-given points
 // k_wave.cu: the slot pool (wavefront.cuh); the march kernel in blocks of 128 or 256 threads; for a
 // spline plan with TMA-staged coefficient bricks (smp_render_opts.spline_bricks) the brick kernel
-WaveFn wf_march_fn(int fk, bool fp64, int block, bool bricks);
+// `copies` of the Bessel table in shared memory: 1, or march_copies(block) where they fit
+constexpr int march_copies(int block) { return block == 256 ? 4 : 2; }
+WaveFn wf_march_fn(int fk, bool fp64, int block, bool bricks, int copies);
 WaveFn wf_event_fn(int fk);
 WaveFn wf_finish_fn(int fk);
 // k_adjoint.cu, adjoint_sweep.cu

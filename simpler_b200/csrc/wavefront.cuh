@@ -32,15 +32,16 @@ namespace smp {
 #define SMP_WF_MARCH_MIN_BLOCKS 6
 #endif
 
-// the state march_step reads and writes
-struct MarchState {
+// the state march_step reads and writes; TAB is how the kernel holds the Bessel table
+template <class TAB> struct MarchStateT {
     float3 mp, md, mg;
     float mn, cur, dist_acc, dlimit, s, mtotf, hh;
     double mtot, cur_d;
     int steps, end, prec, stop;
-    const float4 *tab;
+    TAB tab;
     const Inst *inst;          // batched sweep only
 };
+using MarchState = MarchStateT<const float4 *>;
 
 // the rest of a Lane, stored per slot as one 128-byte record moved with 16-byte accesses
 struct __align__(16) EventPart {
@@ -237,15 +238,29 @@ __device__ __forceinline__ void warp_append2(int *arr, unsigned *c, int n_slots,
 // advance up to `chunk` ER steps each. When fewer slots
 // are live than the grid has lanes, the chunk grows in proportion (up to 64x) so the last photons
 // are not paced by launch latency. F64: the FP64 path-length form (only its accumulator is
-// loaded, carried and stored).
-template <int FK, int F64, int BLOCK>
+// loaded, carried and stored). REP: copies of the Bessel table in shared memory (RepTable).
+template <int REP> struct MarchTable { using T = RepTable<REP>; };
+template <> struct MarchTable<1> { using T = const float4 *; };
+template <int FK, int F64, int BLOCK, int REP>
 __global__ void __launch_bounds__(BLOCK, (FK == FK_SPLINE ? 3 : SMP_WF_MARCH_MIN_BLOCKS) * 128 / BLOCK)
 wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveParams W, int it) {
     extern __shared__ __align__(16) float4 smem_tab[];
     const int lane = threadIdx.x & 31, cur = it & 1, nxt = cur ^ 1;
     const unsigned n0 = list_cnt(W, cur)[0], n = n0 + list_cnt(W, cur)[1];
     if (n == 0u) return;
-    if (FK <= FK_BESSELN) {
+    typename MarchTable<REP>::T tab;
+    if constexpr (REP > 1) {
+        for (int i = threadIdx.x; i < P.field.bnodes; i += BLOCK) {
+            const float4 e = __ldg(P.field.btab + i);
+#pragma unroll
+            for (int r = 0; r < REP; ++r) smem_tab[REP * i + r] = e;
+        }
+        __syncthreads();
+        tab.p = smem_tab + (lane & (REP - 1));
+    } else {
+        tab = FK <= FK_BESSELN ? smem_tab : nullptr;     // the spline: no staged brick, global quads
+    }
+    if (FK <= FK_BESSELN && REP == 1) {
         if (!stage_to_shared(smem_tab, P.field.btab, unsigned(P.field.bnodes) * 16u, P.counters + CNT_STAGE_TIMEOUT)) {
             // timed out (recorded in the counters): copy with plain loads; a late bulk copy
             // writes the same bytes
@@ -264,7 +279,7 @@ wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveP
         int slot = 0;
         if (valid) {
             slot = two_class_at(W.list[cur], n0, W.n_slots, i);
-            MarchState M;
+            MarchStateT<typename MarchTable<REP>::T> M;
             const float4 a = W.ma[slot], b = W.mb[slot], c = W.mc[slot], d = W.mdd[slot];
             const int4 e = W.mi[slot];
             M.mp = f3(a.x, a.y, a.z); M.mn = a.w;
@@ -275,11 +290,10 @@ wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveP
             M.hh = 0.5f * M.cur;
             M.cur_d = double(M.cur);
             M.mtot = F64 ? W.mt[slot] : 0.0;
-            if (FK == FK_BATCH) {
+            M.tab = tab;
+            if constexpr (FK == FK_BATCH) {
                 M.inst = P.insts + __float_as_int(d.w);
                 M.tab = M.inst->field.btab;
-            } else {
-                M.tab = FK == FK_SPLINE ? nullptr : smem_tab;   // no staged brick: global quads
             }
             const int steps0 = M.steps;
             typename Field<FK>::Cache C;
