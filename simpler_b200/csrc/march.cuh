@@ -212,28 +212,6 @@ __device__ __forceinline__ bool propagate_till_sensor(const KParams &P, float3 &
     return true;
 }
 
-// Scene::addEnergyToImage (scene.cpp:782-829) with bilinear sharing (USE_PIXEL_SHARING): one tap,
-// Image3::addEnergy (image.h:320-324) with the bounds check of addPixel (scene.h:305-312).
-// Warp-aggregated: the lanes that reach this call together are grouped by the film address they
-// add to (__match_any_sync through cooperative groups), each group sums its values (in double for
-// the FP64 film) and one lane issues the atomic. A narrow beam's direct light lands on a handful of
-// pixels, where one atomic per lane would serialise on the same address.
-__device__ __forceinline__ void add_pixel(const KParams &P, void *film, int x, int y, int z, float v) {
-    const bool in = x >= 0 && x < P.X && y >= 0 && y < P.Y && z >= 0 && z < P.Z;
-    const size_t i = in ? (size_t(z) * P.Y + y) * P.X + x : 0;
-    const unsigned long long key =
-        in ? reinterpret_cast<unsigned long long>(film) + (unsigned long long)i * (P.fp64 ? 8ull : 4ull) : 0ull;
-    const cg::coalesced_group active = cg::coalesced_threads();
-    const cg::coalesced_group same = cg::labeled_partition(active, key);
-    if (P.fp64) {
-        const double s = cg::reduce(same, double(v), cg::plus<double>());
-        if (in && same.thread_rank() == 0) atomicAdd(reinterpret_cast<double *>(film) + i, s);
-    } else {
-        const float s = cg::reduce(same, v, cg::plus<float>());
-        if (in && same.thread_rank() == 0) atomicAdd(reinterpret_cast<float *>(film) + i, s);
-    }
-}
-
 // Film cell of a splat at sensor point p with path length pl (scene.cpp:782-829) on a film X
 // pixels wide: the bilinear base pixel (ix, iy), its fractions (fx, fy) and the bin iz; false when
 // pl is outside the binned range.
@@ -257,6 +235,50 @@ __device__ __forceinline__ bool splat_bin(const KParams &P, int X, float3 p, dou
     return true;
 }
 
+// Scene::addEnergyToImage (scene.cpp:782-829) with bilinear sharing (USE_PIXEL_SHARING): the four taps
+// of base pixel (ix, iy) in bin iz, each with Image3::addEnergy's bounds check (image.h:320-324,
+// scene.h:305-312). Warp-aggregated: the lanes that splat together and share a base pixel share all four
+// taps, so one match groups them, the group's first lane sums the others' values (in double for the
+// FP64 film) and issues the atomics. A narrow beam's direct light lands on a handful of pixels, where
+// one atomic per lane would serialise on the same address. Most groups are a single lane, which then
+// goes straight to its atomics; a match and a tree reduction per tap took twice the instructions.
+template <class T>
+__device__ __forceinline__ void add_tap(const KParams &P, T *film, int x, int y, int z, T v) {
+    if (x >= 0 && x < P.X && y >= 0 && y < P.Y && z >= 0 && z < P.Z) atomicAdd(film + (size_t(z) * P.Y + y) * P.X + x, v);
+}
+template <class T>
+__device__ __forceinline__ void add_taps_t(const KParams &P, T *film, int ix, int iy, int iz, float v0, float v1, float v2,
+                                           float v3) {
+    // a base pixel none of whose taps can lie on the film
+    if (ix < -1 || ix >= P.X || iy < -1 || iy >= P.Y || iz < 0 || iz >= P.Z) return;
+    const unsigned act = __activemask();
+    const unsigned lane = threadIdx.x & 31u;
+    unsigned same = __match_any_sync(act, ((unsigned long long)iz * unsigned(P.Y + 1) + unsigned(iy + 1)) * unsigned(P.X + 1) + unsigned(ix + 1));
+    if (P.n_inst) same &= __match_any_sync(act, reinterpret_cast<unsigned long long>(film));     // a sweep's films
+    T s0 = T(v0), s1 = T(v1), s2 = T(v2), s3 = T(v3);
+    const bool first = (same & ((1u << lane) - 1u)) == 0u;
+    unsigned rest = first ? same & (same - 1u) : 0u;      // the first lane collects the others
+    while (__any_sync(act, rest != 0u)) {
+        const int src = rest ? __ffs(rest) - 1 : int(lane);
+        const float a = __shfl_sync(act, v0, src), b = __shfl_sync(act, v1, src), c = __shfl_sync(act, v2, src),
+                    d = __shfl_sync(act, v3, src);
+        if (rest) {
+            s0 += T(a); s1 += T(b); s2 += T(c); s3 += T(d);
+            rest &= rest - 1u;
+        }
+    }
+    if (!first) return;
+    add_tap(P, film, ix, iy, iz, s0);
+    add_tap(P, film, ix + 1, iy, iz, s1);
+    add_tap(P, film, ix, iy + 1, iz, s2);
+    add_tap(P, film, ix + 1, iy + 1, iz, s3);
+}
+__device__ __forceinline__ void add_taps(const KParams &P, void *film, int ix, int iy, int iz, float v0, float v1, float v2,
+                                         float v3) {
+    if (P.fp64) add_taps_t(P, static_cast<double *>(film), ix, iy, iz, v0, v1, v2, v3);
+    else add_taps_t(P, static_cast<float *>(film), ix, iy, iz, v0, v1, v2, v3);
+}
+
 __device__ __forceinline__ void splat(Lane &L, const KParams &P, float3 p, double pl, int depth, float val) {
     if (P.records) {
         smp_photon_record *rec = P.records + (L.idx - P.first_photon);
@@ -272,11 +294,8 @@ __device__ __forceinline__ void splat(Lane &L, const KParams &P, float3 p, doubl
     int ix, iy, iz;
     float fx, fy;
     if (!splat_bin(P, P.X, p, pl, depth, ix, iy, iz, fx, fy)) return;
-    void *film = med_film(L, P);
-    add_pixel(P, film, ix, iy, iz, val * (1.0f - fx) * (1.0f - fy));
-    add_pixel(P, film, ix + 1, iy, iz, val * fx * (1.0f - fy));
-    add_pixel(P, film, ix, iy + 1, iz, val * (1.0f - fx) * fy);
-    add_pixel(P, film, ix + 1, iy + 1, iz, val * fx * fy);
+    add_taps(P, med_film(L, P), ix, iy, iz, val * (1.0f - fx) * (1.0f - fy), val * fx * (1.0f - fy),
+             val * (1.0f - fx) * fy, val * fx * fy);
 }
 
 // Henyey-Greenstein (phase.cpp:17-21, :40-76; util.h:17-27)
@@ -686,6 +705,8 @@ struct NoHook {
 template <int FK, class H = NoHook>
 __device__ __forceinline__ int run_events(Lane &L, const KParams &P, int ev, H *h = nullptr) {
     for (;;) {
+        float dlimit = 0.0f;                                    // the march the event starts,
+        bool go = false, at_start = false;                      // if it does, and whether its field is still unknown
         if (ev == EV_MARCH_END) {
             if (!P.fp64) L.mtot = double(L.mtotf);
             if (L.end == 0 && !isfinite((L.mp.x + L.mp.y) + (L.mp.z + L.md.x) + (L.md.y + L.md.z) + L.mn))
@@ -738,105 +759,80 @@ __device__ __forceinline__ int run_events(Lane &L, const KParams &P, int ev, H *
                 L.mtot = L.total;
                 L.first = 1;
                 L.large = med_large(L, P);
-                begin_march<FK>(L, P, L.large, false);
-                if (march_has_steps(L)) return ST_MARCH;
-                ev = EV_MARCH_END;
+                dlimit = L.large;
+                go = true;
             } else {
                 ev = EV_SCATTER;
             }
             break;
         }
         case EV_MARCH_END: {
+            // movePhotonTillSensor (scene.cpp:622-703) for the direct march and connections, movePhoton
+            // (scene.cpp:706-780) for moves; both meet a face here
             const float disy = L.dist_acc;
-            if (L.ctx == CTX_DIRECT || L.ctx == CTX_CONNECT) {
-                // movePhotonTillSensor (scene.cpp:622-703)
+            const bool sensor = L.ctx == CTX_DIRECT || L.ctx == CTX_CONNECT;
+            bool face, hit = false;
+            if (sensor) {
                 if (L.first) { L.d2s = disy; L.first = 0; } else { L.d2s += disy; }
                 L.large -= disy;
-                bool done = false, ok = false;
-                if (L.large < 0.0f) { done = true; ok = false; }
-                else {
-                    float3 n = face_normal(P, L.mp);
-                    if (fabsf(P.cam_dir[0] - n.x) < kEps && fabsf(P.cam_dir[1] - n.y) < kEps &&
-                        fabsf(P.cam_dir[2] - n.z) < kEps) { done = true; ok = true; }
-                    else {
-                        float3 d1 = bsdf_sample(L, P, L.md, n);
-                        if (dot3(d1, n) < 0.0f) {
-                            L.md = d1;
-                            begin_march<FK>(L, P, L.large, false);
-                            if (march_has_steps(L)) return ST_MARCH;
-                            ev = EV_MARCH_END;
-                            break;
-                        }
-                        done = true; ok = false;
-                    }
-                }
-                if (!done) break;
-                if (L.ctx == CTX_DIRECT) {
-                    // directTracing (photon.cpp:41-87); total is the photon's own
-                    L.total = L.mtot;
-                    if (ok) {
-                        float3 d1 = normalized(L.md);
-                        float ior = L.mn;
-                        float3 refr = d1;
-                        float fw = 1.0f;
-                        if (ior > 1.0f) {
-                            refr.x = refr.x / ior;
-                            refr = normalized(refr);
-                            fw = (1.0f - fresnel(d1.x, refr.x, 1.0f / ior)) / ior / ior;
-                        }
-                        float3 p1 = L.mp;
-                        float dts = 0.0f;
-                        if (propagate_till_sensor(P, p1, refr, dts)) {
-                            acc_total(L.total, dts, P.fp64);
-                            float val = med_weight(L, P) * expf(-med_sigma_t(L, P) * L.d2s) * fw;
-                            splat(L, P, p1, L.total, 0, val);
-                            if (H::on) h->splatted(L, p1, L.total, 0, val);
-                        }
-                    }
-                    ev = EV_SCATTER;
-                } else {
-                    // addEnergyInParticle (scene.cpp:866-946); its path length is a copy
-                    if (ok) {
-                        float3 dsen = normalized(L.md);
-                        float ior = L.mn;
-                        float3 refr = dsen;
-                        float fw = 1.0f;
-                        if (ior > 1.0f) {
-                            refr.x = refr.x / ior;
-                            refr = normalized(refr);
-                            fw = (1.0f - fresnel(dsen.x, refr.x, 1.0f / ior)) / ior / ior;
-                        }
-                        float fore = dot3(refr, ld3(P.cam_dir)) / dot3(dsen, ld3(P.cam_dir));
-                        double tot = L.mtot;
-                        float3 p1 = L.mp;
-                        float dts = 0.0f;
-                        if (propagate_till_sensor(P, p1, refr, dts)) {
-                            acc_total(tot, dts, P.fp64);
-                            float val = med_weight(L, P) * 6.28318548202514648f * expf(-med_sigma_t(L, P) * L.d2s) *
-                                        hg_f(med_g(L, P), divs(L.dir, len3(L.dir)), dsen) * fore * fw;
-                            splat(L, P, p1, tot, L.depth, val);
-                            if (H::on) h->splatted(L, p1, tot, L.depth, val);
-                        }
-                    }
-                    ev = EV_SCATTER_ONCE;
-                }
+                face = !(L.large < 0.0f);
             } else {
-                // movePhoton (scene.cpp:706-780)
                 L.rem -= disy;
-                bool ok = true;
-                if (L.rem > kEps) {
-                    float3 n = face_normal(P, L.mp);
-                    float mag = len3(L.md);
-                    float3 d1 = bsdf_sample(L, P, divs(L.md, mag), n);
-                    if (dot3(d1, n) < 0.0f) {
-                        L.md = mul(d1, mag);
-                        begin_march<FK>(L, P, L.rem, false);
-                        if (march_has_steps(L)) return ST_MARCH;
-                        ev = EV_MARCH_END;
+                face = L.rem > kEps;
+            }
+            if (face) {
+                const float3 n = face_normal(P, L.mp);
+                if (sensor && fabsf(P.cam_dir[0] - n.x) < kEps && fabsf(P.cam_dir[1] - n.y) < kEps &&
+                    fabsf(P.cam_dir[2] - n.z) < kEps) {
+                    hit = true;
+                } else {
+                    const float mag = sensor ? 1.0f : len3(L.md);
+                    const float3 d1 = bsdf_sample(L, P, sensor ? L.md : divs(L.md, mag), n);
+                    if (dot3(d1, n) < 0.0f) {                   // reflected: the march goes on
+                        L.md = sensor ? d1 : mul(d1, mag);
+                        dlimit = sensor ? L.large : L.rem;
+                        go = true;
                         break;
                     }
-                    ok = false;
                 }
+            }
+            if (sensor) {
+                // directTracing (photon.cpp:41-87: its path length is the photon's own) and
+                // addEnergyInParticle (scene.cpp:866-946: its path length is a copy)
+                const bool connect = L.ctx == CTX_CONNECT;
+                double tot = L.mtot;
+                if (!connect) L.total = tot;
+                if (hit) {
+                    const float3 dsen = normalized(L.md);
+                    const float ior = L.mn;
+                    float3 refr = dsen;
+                    float fw = 1.0f;
+                    if (ior > 1.0f) {
+                        refr.x = refr.x / ior;
+                        refr = normalized(refr);
+                        fw = (1.0f - fresnel(dsen.x, refr.x, 1.0f / ior)) / ior / ior;
+                    }
+                    const float3 out = refr;                    // before the sensor lens
+                    float3 p1 = L.mp;
+                    float dts = 0.0f;
+                    if (propagate_till_sensor(P, p1, refr, dts)) {
+                        acc_total(tot, dts, P.fp64);
+                        if (!connect) L.total = tot;
+                        float val = med_weight(L, P);
+                        if (connect) val = val * 6.28318548202514648f;
+                        val = val * expf(-med_sigma_t(L, P) * L.d2s);
+                        if (connect) {
+                            const float fore = dot3(out, ld3(P.cam_dir)) / dot3(dsen, ld3(P.cam_dir));
+                            val = val * hg_f(med_g(L, P), divs(L.dir, len3(L.dir)), dsen) * fore;
+                        }
+                        val = val * fw;
+                        splat(L, P, p1, tot, L.depth, val);     // depth 0: direct
+                        if (H::on) h->splatted(L, p1, tot, L.depth, val);
+                    }
+                }
+                ev = connect ? EV_SCATTER_ONCE : EV_SCATTER;
+            } else {
+                const bool ok = !face;                          // else refracted out
                 L.total = L.mtot;
                 L.pos = L.mp;
                 L.dir = L.md;
@@ -845,21 +841,6 @@ __device__ __forceinline__ int run_events(Lane &L, const KParams &P, int ev, H *
                 else ++L.depth;
                 ev = EV_VERTEX;
             }
-            break;
-        }
-        case EV_SCATTER: {
-            if (H::on && h->at(L, EV_SCATTER)) return ST_HOOK;
-            if (!roulette(L, P)) { L.end = SMP_END_NO_SCATTER; ev = EV_FINISH; break; }
-            float dist = -med_mfp(L, P) * logf(draw(L, P));
-            L.ctx = CTX_MOVE_FIRST;
-            L.sampled = dist;
-            L.rem = dist;
-            L.mp = L.pos;
-            L.md = L.dir;
-            L.mtot = L.total;
-            begin_march<FK>(L, P, dist, true);
-            if (march_has_steps(L)) return ST_MARCH;
-            ev = EV_MARCH_END;
             break;
         }
         case EV_VERTEX: {
@@ -876,29 +857,33 @@ __device__ __forceinline__ int run_events(Lane &L, const KParams &P, int ev, H *
                 L.mtot = L.total;
                 L.first = 1;
                 L.large = med_large(L, P);
-                begin_march<FK>(L, P, L.large, false);
-                if (march_has_steps(L)) return ST_MARCH;
-                ev = EV_MARCH_END;
+                dlimit = L.large;
+                go = true;
                 break;
             }
             ev = EV_SCATTER_ONCE;
             break;
         }
+        case EV_SCATTER:
         case EV_SCATTER_ONCE: {
-            if (H::on && h->at(L, EV_SCATTER_ONCE)) return ST_HOOK;
-            if (!roulette(L, P)) { L.end = SMP_END_ABSORBED; ev = EV_FINISH; break; }
-            float mag = len3(L.dir);
-            float3 d1 = hg_sample(L, P, divs(L.dir, mag));
-            L.dir = mul(d1, mag);
-            float dist = -med_mfp(L, P) * logf(draw(L, P));
-            L.ctx = CTX_MOVE_VERTEX;
+            const bool once = ev == EV_SCATTER_ONCE;            // at a vertex: a new direction
+            if (H::on && h->at(L, ev)) return ST_HOOK;
+            if (!roulette(L, P)) { L.end = once ? SMP_END_ABSORBED : SMP_END_NO_SCATTER; ev = EV_FINISH; break; }
+            if (once) {
+                const float mag = len3(L.dir);
+                const float3 d1 = hg_sample(L, P, divs(L.dir, mag));
+                L.dir = mul(d1, mag);
+            }
+            const float dist = -med_mfp(L, P) * logf(draw(L, P));
+            L.ctx = once ? CTX_MOVE_VERTEX : CTX_MOVE_FIRST;
+            if (!once) L.sampled = dist;
             L.rem = dist;
             L.mp = L.pos;
             L.md = L.dir;
             L.mtot = L.total;
-            begin_march<FK>(L, P, dist, true);
-            if (march_has_steps(L)) return ST_MARCH;
-            ev = EV_MARCH_END;
+            dlimit = dist;
+            go = true;
+            at_start = true;
             break;
         }
         default: {   // EV_FINISH
@@ -916,6 +901,12 @@ __device__ __forceinline__ int run_events(Lane &L, const KParams &P, int ev, H *
             }
             return ST_FETCH;
         }
+        }
+        // one march start for every event: the lanes of a warp meet here, and the code is there once
+        if (go) {
+            begin_march<FK>(L, P, dlimit, at_start);
+            if (march_has_steps(L)) return ST_MARCH;
+            ev = EV_MARCH_END;
         }
     }
 }
