@@ -347,6 +347,11 @@ int smp_trace_photons(const smp_scene_desc *scene, const smp_medium_desc *medium
 int smp_field_eval(const smp_field_desc *field, double scaling, int64_t n_points,
                    const double *points, double *n_out, double *grad_out);
 
+/* n(p) alone at n_points host points: smp_field_eval's n_out bit for bit. For the point-source field
+   a kernel of its own does without the gradient's work. */
+int smp_field_values(const smp_field_desc *field, double scaling, int64_t n_points,
+                     const double *points, double *n_out);
+
 /* Texture CDF exactly as area_textured_source builds it (float accumulate + normalise),
    tex_x*tex_y+1 entries. */
 int smp_texture_cdf(const double *texture, int32_t tex_x, int32_t tex_y, float *cdf_out);

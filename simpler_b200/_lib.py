@@ -165,7 +165,7 @@ EXPORTS = [
     "smp_plan_read_image", "smp_plan_film", "smp_plan_stats", "smp_plan_render", "smp_trace_photons",
     "smp_field_eval", "smp_texture_cdf", "smp_spline_prefilter", "smp_render_batch", "smp_fp32_peak",
     "smp_render_noalloc", "smp_adjoint_param_count", "smp_plan_adjoint", "smp_render_adjoint", "smp_plan_tune",
-    "smp_batch_tune_steps", "smp_plan_tune_step",
+    "smp_batch_tune_steps", "smp_plan_tune_step", "smp_field_values",
 ]
 
 _lib = None
@@ -205,6 +205,7 @@ def load() -> C.CDLL:
     lib.smp_trace_photons.argtypes = [P(SceneDesc), P(MediumDesc), P(FieldDesc), P(RenderOpts), C.c_int64,
                                       C.c_int64, C.c_int64, vp, vp, P(PhotonRecord), vp]
     lib.smp_field_eval.argtypes = [P(FieldDesc), C.c_double, C.c_int64, vp, vp, vp]
+    lib.smp_field_values.argtypes = [P(FieldDesc), C.c_double, C.c_int64, vp, vp]
     lib.smp_texture_cdf.argtypes = [vp, C.c_int32, C.c_int32, vp]
     lib.smp_spline_prefilter.argtypes = [vp, vp, vp]
     lib.smp_render_batch.argtypes = [P(SceneDesc), P(InstanceDesc), C.c_int32, P(RenderOpts), vp, P(Stats)]

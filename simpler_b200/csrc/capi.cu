@@ -1604,6 +1604,49 @@ int smp_field_eval(const smp_field_desc *field, double scaling, int64_t n_points
     return SMP_OK;
 }
 
+int smp_field_values(const smp_field_desc *field, double scaling, int64_t n_points, const double *points, double *n_out) {
+    if (!field || n_points < 0 || (n_points > 0 && (!points || !n_out))) return set_error(SMP_ERR_BAD_ARG, "bad arguments");
+    int fk;
+    int rc = field_kind(*field, &fk);
+    if (rc) return rc;
+    const int nt = field->theta_sources, block = sources_values_block();
+    const size_t smem = size_t((nt + 3) / 4) * size_t(block) * sizeof(float4);
+    // other kinds, and rows longer than the shared memory holds (440 places): the probe, its gradient dropped
+    if (fk != FK_SOURCES || smem > 220 * 1024) {
+        std::vector<double> g(size_t(n_points) * 3);
+        return smp_field_eval(field, scaling, n_points, points, n_out, g.data());
+    }
+    rc = check_device(0);
+    if (rc) return rc;
+    if (n_points == 0) return SMP_OK;
+    FieldParams F;
+    fill_field_params(*field, fk, F);
+    std::vector<float4> c;
+    source_centres(*field, c);
+    const ValuesFn fn = sources_values_fn();
+    rc = allow_dynamic_smem(reinterpret_cast<const void *>(fn), smem);
+    if (rc) return rc;
+    const size_t np = size_t(n_points);
+    float4 *d_cen = nullptr;
+    double *d_pts = nullptr, *d_n = nullptr;
+    cudaError_t e = cudaMalloc(&d_cen, c.size() * sizeof(float4));
+    if (e == cudaSuccess) e = cudaMalloc(&d_pts, np * 3 * sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc(&d_n, np * sizeof(double));
+    if (e == cudaSuccess) e = cudaMemcpy(d_cen, c.data(), c.size() * sizeof(float4), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d_pts, points, np * 3 * sizeof(double), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        F.centers = d_cen;
+        fn<<<unsigned((np + block - 1) / block), block, smem>>>(F, nt, n_points, d_pts, d_n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(n_out, d_n, np * sizeof(double), cudaMemcpyDeviceToHost);
+    cudaFree(d_cen);
+    cudaFree(d_pts);
+    cudaFree(d_n);
+    if (e != cudaSuccess) return set_error(SMP_ERR_CUDA, "field values: %s", cudaGetErrorString(e));
+    return SMP_OK;
+}
+
 // FP32 FMA throughput probe: every thread runs eight independent FMA chains.
 __global__ void fp32_peak_kernel(float *out, int iters) {
     float a[8];

@@ -14,6 +14,7 @@ struct AdjParams;
 typedef void (*MarchFn)(KParams);
 typedef void (*WaveFn)(KParams, WaveParams, int);
 typedef void (*ProbeFn)(FieldParams, float, long long, const double *, double *, double *);
+typedef void (*ValuesFn)(FieldParams, int, long long, const double *, double *);
 typedef void (*AdjFn)(KParams, AdjParams);
 typedef void (*AdjRoundFn)(KParams, AdjParams, int);
 typedef void (*AdjWaveFn)(KParams, WaveParams, AdjParams, int);
@@ -22,6 +23,8 @@ typedef void (*AdjWaveFn)(KParams, WaveParams, AdjParams, int);
 MarchFn march_fn(int fk);                        // persistent lane loop (march.cuh)
 MarchFn plain_fn(int fk);                        // one thread per photon (plain.cuh)
 ProbeFn field_probe_fn(int fk);                  // field at host-given points
+ValuesFn sources_values_fn();                    // n alone of the point sources, (nt + 3) / 4 * block * 16
+int sources_values_block();                      // bytes of dynamic shared memory, blocks of this size
 // k_wave.cu: the slot pool (wavefront.cuh); the march kernel in blocks of 128 or 256 threads; for a
 // spline plan with TMA-staged coefficient bricks (smp_render_opts.spline_bricks) the brick kernel
 // `copies` of the Bessel table in shared memory: 1, or march_copies(block) where they fit

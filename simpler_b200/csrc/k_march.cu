@@ -35,6 +35,9 @@ MarchFn plain_fn(int fk) {
     }
 }
 
+ValuesFn sources_values_fn() { return sources_values_kernel; }
+int sources_values_block() { return kValuesBlock; }
+
 ProbeFn field_probe_fn(int fk) {
     switch (fk) {
         case FK_BESSEL0: return field_probe_kernel<FK_BESSEL0>;

@@ -353,14 +353,16 @@ def sources_to_spline(setup: Setup, n: int = 96, margin: int = 6) -> Setup:
     h = (hi - lo) / (n - 1 - 2 * margin)
     lo, hi = lo - margin * h, hi + margin * h
     axes = [np.linspace(lo[i], hi[i], n) for i in range(3)]
-    z, y, x = np.meshgrid(axes[2], axes[1], axes[0], indexing="ij")
-    pts = np.stack([x.ravel(), y.ravel(), z.ravel()], axis=1)
+    pts = np.empty((n, n, n, 3))
+    pts[..., 0], pts[..., 1], pts[..., 2] = axes[0], axes[1][:, None], axes[2][:, None, None]
     # dn = n - n_o at the nodes (n_o = 0 keeps dn's own float precision), no gating at the nodes
     probe = dataclasses.replace(setup, n_o=0.0, emitter_gap=-1e-3, sensor_gap=-1e-3)
-    vals, _ = field_eval(probe, 0.0, pts)
-    samples = np.ascontiguousarray(vals.reshape(n, n, n), dtype=np.float32)
-    coeff = np.zeros_like(samples)
+    lib, fd = L.load(), probe.field_desc()
+    vals = np.empty((n, n, n))
+    L.check(lib.smp_field_values(C.byref(fd), 0.0, n ** 3, _ptr(pts), _ptr(vals)))
+    samples = vals.astype(np.float32)
+    coeff = np.empty_like(samples)
     dims = np.array([n, n, n], dtype=np.int32)
-    L.check(L.load().smp_spline_prefilter(_ptr(samples), _ptr(dims), _ptr(coeff)))
+    L.check(lib.smp_spline_prefilter(_ptr(samples), _ptr(dims), _ptr(coeff)))
     return dataclasses.replace(setup, field_type=L.FIELD_SPLINE, grid_coeff=coeff, grid_offset=float(setup.n_o),
                                grid_min=tuple(float(v) for v in lo), grid_max=tuple(float(v) for v in hi))
