@@ -90,39 +90,52 @@ static int cdf_guide(const std::vector<float> &cdf, std::vector<int> &guide) {
 
 // Spline<3>::build1d (renderer/include/spline.h:686-714): causal + anticausal recursive filter,
 // pole z1 = sqrt(3) - 2, mirror boundary.
-static void prefilter_1d(const float *data, long off, long stride, int size, float *out) {
+// pw[i] = z1^i in float, i < 2 size - 2, shared by all lines of an axis.
+static std::vector<float> prefilter_powers(int size) {
     const float z1 = -2.0f + std::sqrt(3.0f);
-    std::vector<float> cp(size), cn(size);
+    std::vector<float> pw(size_t(std::max(1, 2 * size - 2)));
+    for (size_t i = 0; i < pw.size(); ++i) pw[i] = float(std::pow(double(z1), double(i)));
+    return pw;
+}
+static void prefilter_1d(const float *data, long off, long stride, int size, const float *pw, float *cp, float *out) {
+    const float z1 = -2.0f + std::sqrt(3.0f);
     float c0 = 0.0f;
-    for (int i = 0; i < size; ++i) c0 += data[off + i * stride] * float(std::pow(double(z1), i));
-    for (int i = size - 2; i > 0; --i) c0 += data[off + i * stride] * float(std::pow(double(z1), 2 * size - 2 - i));
+    for (int i = 0; i < size; ++i) c0 += data[off + i * stride] * pw[i];
+    for (int i = size - 2; i > 0; --i) c0 += data[off + i * stride] * pw[2 * size - 2 - i];
     c0 /= float(1.0 - std::pow(double(z1), 2 * size - 2));
     cp[0] = c0;
     for (int i = 1; i < size; ++i) cp[i] = data[off + i * stride] + z1 * cp[i - 1];
-    cn[size - 1] = z1 / (z1 * z1 - 1.0f) * (cp[size - 1] + z1 * cp[size - 2]);
-    for (int i = size - 2; i >= 0; --i) cn[i] = z1 * (cn[i + 1] - cp[i]);
-    for (int i = 0; i < size; ++i) out[i] = 6.0f * cn[i];
+    // the anticausal pass in place of cn: out[i] = 6 cn[i], cn kept one ahead
+    float cn = z1 / (z1 * z1 - 1.0f) * (cp[size - 1] + z1 * cp[size - 2]);
+    out[size - 1] = 6.0f * cn;
+    for (int i = size - 2; i >= 0; --i) {
+        cn = z1 * (cn - cp[i]);
+        out[i] = 6.0f * cn;
+    }
 }
 
-// Spline<3>::build3d (spline.h:739-764): y, then x, then z passes
+template <class F> static void host_parallel(size_t n, F f);
+
+// Spline<3>::build3d (spline.h:739-764): y, then x, then z passes; the lines of a pass are independent
+// and run on the host's threads
 static void prefilter_3d(const float *samples, const int N[3], float *coeff) {
     const long s01 = long(N[0]) * N[1];
-    std::vector<float> tmp(std::max(std::max(N[0], N[1]), N[2]));
-    for (int k = 0; k < N[2]; ++k)
-        for (int i = 0; i < N[0]; ++i) {
-            prefilter_1d(samples, k * s01 + i, N[0], N[1], tmp.data());
-            for (int t = 0; t < N[1]; ++t) coeff[i + t * N[0] + k * s01] = tmp[t];
-        }
-    for (int k = 0; k < N[2]; ++k)
-        for (int j = 0; j < N[1]; ++j) {
-            prefilter_1d(coeff, k * s01 + long(j) * N[0], 1, N[0], tmp.data());
-            for (int t = 0; t < N[0]; ++t) coeff[t + j * N[0] + k * s01] = tmp[t];
-        }
-    for (int i = 0; i < N[0]; ++i)
-        for (int j = 0; j < N[1]; ++j) {
-            prefilter_1d(coeff, long(j) * N[0] + i, s01, N[2], tmp.data());
-            for (int t = 0; t < N[2]; ++t) coeff[i + j * N[0] + t * s01] = tmp[t];
-        }
+    auto pass = [&](const float *src, int axis, int other, long sa, long s1, int outer, long s2) {
+        // lines along `axis` of stride sa: `outer` planes of stride s2, N[other] lines of stride s1
+        const int size = N[axis];
+        const std::vector<float> pw = prefilter_powers(size);
+        host_parallel(size_t(outer) * N[other], [&, size](size_t a, size_t b) {
+            std::vector<float> tmp(2 * size_t(size));
+            for (size_t l = a; l < b; ++l) {
+                const long off = long(l / N[other]) * s2 + long(l % N[other]) * s1;
+                prefilter_1d(src, off, sa, size, pw.data(), tmp.data(), tmp.data() + size);
+                for (int t = 0; t < size; ++t) coeff[off + t * sa] = tmp[size + t];
+            }
+        });
+    };
+    pass(samples, 1, 0, N[0], 1, N[2], s01);
+    pass(coeff, 0, 1, 1, N[0], N[2], s01);
+    pass(coeff, 2, 0, s01, 1, N[1], N[0]);
 }
 
 // rif_sources::recompute_derived_ (renderer/include/rif_sources.h:156-198): centres of the
