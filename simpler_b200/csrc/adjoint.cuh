@@ -297,6 +297,10 @@ template <int NW> struct FieldAdjPW {
             }
         }
     }
+    static __device__ __forceinline__ void eval_s(const FieldParams &F, float3 p, float tau, float &n, float3 &g, float H[6],
+                                                  Cache &k, Acc &) {
+        eval_h(F, p, tau, n, g, H, k);
+    }
     static __device__ __forceinline__ void theta_c(const FieldParams &F, float3, float, float a, float3 b, Acc &c,
                                                    const AdjParams &, const Cache &k) {
         if (k.gap) return;
@@ -335,20 +339,15 @@ __device__ __forceinline__ void bspline_dd(float t, float dd[4]) {
     dd[3] = f;
 }
 template <> struct FieldAdj<FK_SPLINE> {
-    struct Acc {};
+    struct Acc { SplineCell C; };              // the tap rows of the sweep's current cell
     struct Cache {};
     static __device__ __forceinline__ void begin(Acc &, Lane &, const KParams &, float) {}
-    static __device__ __forceinline__ void clear(Acc &) {}
+    static __device__ __forceinline__ void clear(Acc &c) { c.C.clear(); }
     static __device__ __forceinline__ void taps(const FieldParams &F, float3 p, float wx[4], float wy[4], float wz[4],
                                                 float dx[4], float dy[4], float dz[4], float ddx[4], float ddy[4],
                                                 float ddz[4], int ix[4], int iy[4], int iz[4]) {
         const float t0 = (p.x - F.xmin[0]) * F.xres[0], t1 = (p.y - F.xmin[1]) * F.xres[1], t2 = (p.z - F.xmin[2]) * F.xres[2];
-        bspline_weights(t0, wx, dx);
-        bspline_weights(t1, wy, dy);
-        bspline_weights(t2, wz, dz);
-        bspline_dd(t0, ddx);
-        bspline_dd(t1, ddy);
-        bspline_dd(t2, ddz);
+        weights(t0, t1, t2, wx, wy, wz, dx, dy, dz, ddx, ddy, ddz);
         const int bx = int(floorf(t0)) - 1, by = int(floorf(t1)) - 1, bz = int(floorf(t2)) - 1;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -357,35 +356,54 @@ template <> struct FieldAdj<FK_SPLINE> {
             iz[q] = spline_wrap(bz + q, F.N[2]) * F.N[0] * F.N[1];
         }
     }
-    static __device__ __forceinline__ void eval_h(const FieldParams &F, float3 p, float, float &n, float3 &g, float H[6]) {
+    static __device__ __forceinline__ void weights(float t0, float t1, float t2, float wx[4], float wy[4], float wz[4],
+                                                   float dx[4], float dy[4], float dz[4], float ddx[4], float ddy[4],
+                                                   float ddz[4]) {
+        bspline_weights(t0, wx, dx);
+        bspline_weights(t1, wy, dy);
+        bspline_weights(t2, wz, dz);
+        bspline_dd(t0, ddx);
+        bspline_dd(t1, ddy);
+        bspline_dd(t2, ddz);
+    }
+    // The sixteen rows come in one batch of independent loads, and in the sweep, where a cell's points
+    // follow one another, once per cell (SplineCell): loaded row by row behind a test each, they were a
+    // sweep's whole time (26 of 27 cycles per instruction waiting for them).
+    static __device__ __forceinline__ void eval_s(const FieldParams &F, float3 p, float, float &n, float3 &g, float H[6],
+                                                  Cache &, Acc &acc) {
 #pragma unroll
         for (int j = 0; j < 6; ++j) H[j] = 0.0f;
         if (in_gap(F, p)) { n = F.n_o; g = f3(0.0f, 0.0f, 0.0f); return; }
+        const float t0 = (p.x - F.xmin[0]) * F.xres[0], t1 = (p.y - F.xmin[1]) * F.xres[1], t2 = (p.z - F.xmin[2]) * F.xres[2];
         float wx[4], wy[4], wz[4], dx[4], dy[4], dz[4], ddx[4], ddy[4], ddz[4];
-        int ix[4], iy[4], iz[4];
-        taps(F, p, wx, wy, wz, dx, dy, dz, ddx, ddy, ddz, ix, iy, iz);
+        weights(t0, t1, t2, wx, wy, wz, dx, dy, dz, ddx, ddy, ddz);
+        SplineCell &C = acc.C;
+        const int x = int(floorf(t0)), y = int(floorf(t1)), z = int(floorf(t2));
+        if ((x != C.x) | (y != C.y) | (z != C.z)) {
+            if (spline_on_quads(F, x, y, z)) {
+                spline_rows(F, x, y, z, C.q);
+            } else {
+                int ix[4];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) ix[a] = spline_wrap(x - 1 + a, F.N[0]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int b = 0; b < 4; ++b) {
+                        const float *row = F.coeff + spline_wrap(z - 1 + c, F.N[2]) * F.N[0] * F.N[1] +
+                                           spline_wrap(y - 1 + b, F.N[1]) * F.N[0];
+                        C.q[4 * c + b] = make_float4(__ldg(row + ix[0]), __ldg(row + ix[1]), __ldg(row + ix[2]), __ldg(row + ix[3]));
+                    }
+            }
+            C.x = x; C.y = y; C.z = z;
+        }
         float v = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
         float hxx = 0.0f, hyy = 0.0f, hzz = 0.0f, hxy = 0.0f, hxz = 0.0f, hyz = 0.0f;
-        const int fx = int(floorf((p.x - F.xmin[0]) * F.xres[0]));
-        const bool quad = F.coeff4 != nullptr && unsigned(fx) < unsigned(F.N[0]);
-        int ry[4], rz[4];                                   // the quads' rows
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            ry[q] = iy[q] + 2 * spline_wrap(int(floorf((p.y - F.xmin[1]) * F.xres[1])) - 1 + q, F.N[1]);
-            rz[q] = iz[q] + 2 * F.N[1] * spline_wrap(int(floorf((p.z - F.xmin[2]) * F.xres[2])) - 1 + q, F.N[2]);
-        }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                float r0, r1, r2, r3;
-                if (quad) {
-                    const float4 q = __ldg(F.coeff4 + (rz[c] + ry[b] + fx));
-                    r0 = q.x; r1 = q.y; r2 = q.z; r3 = q.w;
-                } else {
-                    const float *row = F.coeff + iz[c] + iy[b];
-                    r0 = __ldg(row + ix[0]); r1 = __ldg(row + ix[1]); r2 = __ldg(row + ix[2]); r3 = __ldg(row + ix[3]);
-                }
+                const float r0 = C.q[4 * c + b].x, r1 = C.q[4 * c + b].y, r2 = C.q[4 * c + b].z, r3 = C.q[4 * c + b].w;
                 const float sv = r0 * wx[0] + r1 * wx[1] + r2 * wx[2] + r3 * wx[3];
                 const float sd = r0 * dx[0] + r1 * dx[1] + r2 * dx[2] + r3 * dx[3];
                 const float sdd = r0 * ddx[0] + r1 * ddx[1] + r2 * ddx[2] + r3 * ddx[3];
@@ -401,6 +419,12 @@ template <> struct FieldAdj<FK_SPLINE> {
         g = f3(gx * r0, gy * r1, gz * r2);
         H[0] = hxx * r0 * r0; H[1] = hyy * r1 * r1; H[2] = hzz * r2 * r2;
         H[3] = hxy * r0 * r1; H[4] = hxz * r0 * r2; H[5] = hyz * r1 * r2;
+    }
+    static __device__ __forceinline__ void eval_h(const FieldParams &F, float3 p, float s, float &n, float3 &g, float H[6]) {
+        Acc a;
+        a.C.clear();
+        Cache k;
+        eval_s(F, p, s, n, g, H, k, a);
     }
     static __device__ __forceinline__ void theta(const FieldParams &F, float3 p, float, float a, float3 b, Acc &, const AdjParams &A) {
         if (in_gap(F, p)) return;
@@ -419,10 +443,6 @@ template <> struct FieldAdj<FK_SPLINE> {
                 for (int i = 0; i < 4; ++i) atomicAdd(row + ix[i], double(ar * wx[i] + br * dx[i]));
             }
         }
-    }
-    static __device__ __forceinline__ void eval_h(const FieldParams &F, float3 p, float s, float &n, float3 &g, float H[6],
-                                                  Cache &) {
-        eval_h(F, p, s, n, g, H);
     }
     static __device__ __forceinline__ void theta_c(const FieldParams &F, float3 p, float s, float a, float3 b, Acc &c,
                                                    const AdjParams &A, const Cache &) {
@@ -492,6 +512,10 @@ template <int M> struct FieldAdjBessel {
     }
     static __device__ __forceinline__ void eval_h(const FieldParams &F, float3 p, float s, float &n, float3 &g, float H[6]) {
         Cache k;
+        eval_h(F, p, s, n, g, H, k);
+    }
+    static __device__ __forceinline__ void eval_s(const FieldParams &F, float3 p, float s, float &n, float3 &g, float H[6],
+                                                  Cache &k, Acc &) {
         eval_h(F, p, s, n, g, H, k);
     }
     static __device__ __forceinline__ void theta_c(const FieldParams &, float3, float, float a, float3 b, Acc &c,
@@ -696,7 +720,7 @@ __device__ __forceinline__ void sweep_begin(Sweep &w, const KParams &P, const Ad
     float n_k, H[6];
     float3 g_k;
     typename FA::Cache kc;
-    FA::eval_h(F, pk, s, n_k, g_k, H, kc);
+    FA::eval_s(F, pk, s, n_k, g_k, H, kc, acc);
     const float3 u = divs(md_end, n_k);
     const float At = dot3(u, Pa) + dot3(g_k, Da) + dot3(g_k, u) * a_end;
     if (face_end) {
@@ -733,7 +757,7 @@ __device__ __forceinline__ int sweep_point(Sweep &w, const KParams &P, const Adj
     float n1, H[6];
     float3 g1;
     typename FA::Cache kc;
-    FA::eval_h(F, pp, s, n1, g1, H, kc);
+    FA::eval_s(F, pp, s, n1, g1, H, kc, acc);
     const float3 dh = sub(w.d, mul(w.gk, hh));
     const float3 dprev = sub(dh, mul(g1, hh));
     const float q = c / n1;

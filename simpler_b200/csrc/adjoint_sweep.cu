@@ -18,7 +18,7 @@ AdjRoundFn adjoint_sweep_fn(int fk, int n_waves) {
         case FK_BESSEL2: return adjoint_sweep_kernel<FK_BESSEL2, SMP_MAX_WAVES, 4>;
         case FK_PLANEWAVE:
             return n_waves <= 2 ? adjoint_sweep_kernel<FK_PLANEWAVE, 2, 4> : adjoint_sweep_kernel<FK_PLANEWAVE, SMP_MAX_WAVES, 3>;
-        case FK_SPLINE: return adjoint_sweep_kernel<FK_SPLINE, SMP_MAX_WAVES, 3>;
+        case FK_SPLINE: return adjoint_sweep_kernel<FK_SPLINE, SMP_MAX_WAVES, 2>;
         default: return nullptr;
     }
 }
