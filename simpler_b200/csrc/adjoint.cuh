@@ -708,6 +708,26 @@ struct Sweep {
     float T, a0, n0;
 };
 
+// The start of a backward sweep at the segment's end point pk (entry step size h_end), where the field is
+// (n_k, g_k, H): the face's shift, the second kick of the last step and the end point's own use of n.
+// Leaves the sweep's state in w and the end point's cotangent of grad n in b (that of n is a_end).
+__device__ __forceinline__ void sweep_begin_at(Sweep &w, const KParams &P, float3 pk, float h_end, float n_k, float3 g_k,
+                                               const float H[6], float3 md_end, float3 Pa, float3 Da, float a_end, float T,
+                                               bool face_end, float3 &b) {
+    const float3 u = divs(md_end, n_k);
+    const float At = dot3(u, Pa) + dot3(g_k, Da) + dot3(g_k, u) * a_end;
+    if (face_end) {
+        const int ax = face_axis(face_normal(P, pk));
+        add_axis(Pa, ax, -(At + T) / comp(u, ax));
+    } else {
+        T = -At;        // each earlier face crossing delays the sampled end by its own shift
+    }
+    // second kick of the last step, and the end point's own use of n
+    b = mul(Da, 0.5f * h_end);
+    Pa = add(Pa, add(mul(g_k, a_end), hmul(H, b)));
+    w.d = md_end; w.gk = g_k; w.Pa = Pa; w.Da = Da; w.T = T;
+}
+
 template <int FK, class FA>
 __device__ __forceinline__ void sweep_begin(Sweep &w, const KParams &P, const AdjParams &A, long long base, int nent,
                                             float3 md_end, float3 Pa, float3 Da, float a_end, float T, bool face_end,
@@ -718,52 +738,25 @@ __device__ __forceinline__ void sweep_begin(Sweep &w, const KParams &P, const Ad
     w.pn = traj_get(A, base, w.i - 1);          // nent >= 2
     const float3 pk = f3(w.e.x, w.e.y, w.e.z);
     float n_k, H[6];
-    float3 g_k;
+    float3 g_k, b;
     typename FA::Cache kc;
     FA::eval_s(F, pk, s, n_k, g_k, H, kc, acc);
-    const float3 u = divs(md_end, n_k);
-    const float At = dot3(u, Pa) + dot3(g_k, Da) + dot3(g_k, u) * a_end;
-    if (face_end) {
-        const int ax = face_axis(face_normal(P, pk));
-        add_axis(Pa, ax, -(At + T) / comp(u, ax));
-    } else {
-        T = -At;        // each earlier face crossing delays the sampled end by its own shift
-    }
-    // second kick of the last step, and the end point's own use of n
-    const float3 b = mul(Da, 0.5f * w.e.w);
-    Pa = add(Pa, add(mul(g_k, a_end), hmul(H, b)));
+    sweep_begin_at(w, P, pk, w.e.w, n_k, g_k, H, md_end, Pa, Da, a_end, T, face_end, b);
     FA::theta_c(F, pk, s, a_end, b, acc, A, kc);
-    w.d = md_end; w.gk = g_k; w.Pa = Pa; w.Da = Da; w.T = T;
 }
 
-// Undo one step. 0: more to go; 1: the start point is reached (outputs in w); 2: malformed.
-template <int FK, class FA>
-__device__ __forceinline__ int sweep_point(Sweep &w, const KParams &P, const AdjParams &A, long long base, float s,
-                                           typename FA::Acc &acc) {
-    const FieldParams &F = P.field;
-    const float c = w.e.w, hh = 0.5f * c;
-    int j = w.i - 1;
-    if (j < 0) return 2;
-    float4 pe = w.pn;
-    const bool junction = pe.w < 0.0f;
-    if (junction) {
-        j -= 1;
-        if (j < 0) return 2;
-        pe = traj_get(A, base, j);
-    }
-    // the next call's entry, in flight while this step is undone
-    const float4 nx = (j >= 1 && pe.w != 0.0f) ? traj_get(A, base, j - 1) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const float3 pp = f3(pe.x, pe.y, pe.z);
-    float n1, H[6];
-    float3 g1;
-    typename FA::Cache kc;
-    FA::eval_s(F, pp, s, n1, g1, H, kc, acc);
+// Undo one step of size c that started at pp, where the field is (n1, g1, H); pe_w is pp's own entry step
+// size (0: the segment's start point). Leaves the point's cotangents of n and grad n in a1, b1 (at the
+// start point without the second kick of a previous step, there is none).
+__device__ __forceinline__ void sweep_update(Sweep &w, const KParams &P, float c, float3 pp, float pe_w, bool junction, float n1,
+                                             float3 g1, const float H[6], float &a1, float3 &b1) {
+    const float hh = 0.5f * c;
     const float3 dh = sub(w.d, mul(w.gk, hh));
     const float3 dprev = sub(dh, mul(g1, hh));
     const float q = c / n1;
     const float3 Dh = add(w.Da, mul(w.Pa, q));
-    const float a1 = -(q / n1) * dot3(dh, w.Pa);
-    float3 b1 = mul(Dh, hh);
+    a1 = -(q / n1) * dot3(dh, w.Pa);
+    b1 = mul(Dh, hh);
     float3 Pa = add(w.Pa, add(mul(g1, a1), hmul(H, b1)));
     float3 Da = Dh;
     float3 d = dprev;
@@ -779,16 +772,41 @@ __device__ __forceinline__ int sweep_point(Sweep &w, const KParams &P, const Adj
     }
     w.gk = g1;
     w.d = d;
-    if (pe.w == 0.0f) {                // the segment's start point
+    if (pe_w == 0.0f) {                // the segment's start point
         w.Pa = Pa; w.Da = Da; w.a0 = a1; w.b0 = b1; w.n0 = n1;
-        return 1;
+        return;
     }
     // second kick of the previous step
-    const float3 b2 = mul(Da, 0.5f * pe.w);
+    const float3 b2 = mul(Da, 0.5f * pe_w);
     Pa = add(Pa, hmul(H, b2));
     b1 = add(b1, b2);
-    FA::theta_c(F, pp, s, a1, b1, acc, A, kc);
     w.Pa = Pa; w.Da = Da;
+}
+
+// Undo one step. 0: more to go; 1: the start point is reached (outputs in w); 2: malformed.
+template <int FK, class FA>
+__device__ __forceinline__ int sweep_point(Sweep &w, const KParams &P, const AdjParams &A, long long base, float s,
+                                           typename FA::Acc &acc) {
+    const FieldParams &F = P.field;
+    int j = w.i - 1;
+    if (j < 0) return 2;
+    float4 pe = w.pn;
+    const bool junction = pe.w < 0.0f;
+    if (junction) {
+        j -= 1;
+        if (j < 0) return 2;
+        pe = traj_get(A, base, j);
+    }
+    // the next call's entry, in flight while this step is undone
+    const float4 nx = (j >= 1 && pe.w != 0.0f) ? traj_get(A, base, j - 1) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float3 pp = f3(pe.x, pe.y, pe.z);
+    float n1, a1, H[6];
+    float3 g1, b1;
+    typename FA::Cache kc;
+    FA::eval_s(F, pp, s, n1, g1, H, kc, acc);
+    sweep_update(w, P, w.e.w, pp, pe.w, junction, n1, g1, H, a1, b1);
+    if (pe.w == 0.0f) return 1;
+    FA::theta_c(F, pp, s, a1, b1, acc, A, kc);
     w.i = j;
     w.e = pe;
     w.pn = nx;
@@ -1215,10 +1233,312 @@ enum AdjJob : int { JOB_CONN = 1, JOB_MOVE = 2, JOB_DIRECT = 3, JOB_SOURCE = 4 }
 
 
 
+// One photon's backward pass: its jobs in order (connection K, move K, ..., move 1, direct, source) and
+// what they carry, the adjoint (lp, ld) of the photon's position and direction.
+struct PhotonJobs {
+    int job, kv;
+    float s;
+    float3 lp, ld, Ddir;
+    const AdjVertex *V;
+    const AdjSeg *segs;
+};
+struct JobSweep {
+    int c;                     // the job's segment
+    float3 Pa, Da;
+    float a_end, T;
+    bool face_end;
+};
+__device__ __forceinline__ void job_photon(PhotonJobs &J, const AdjParams &A, const AdjPhoton &r) {
+    J.s = r.s;
+    J.V = A.pool + r.off;
+    J.segs = A.segs + 2LL * r.off;
+    J.lp = J.ld = f3(0.0f, 0.0f, 0.0f);
+    J.kv = r.nv - 1;
+    J.job = J.kv >= 1 ? JOB_CONN : JOB_DIRECT;
+}
+__device__ __forceinline__ void job_next(PhotonJobs &J) {
+    if (J.job == JOB_CONN) J.job = JOB_MOVE;
+    else if (J.job == JOB_MOVE) {
+        if (J.kv == 1) J.job = JOB_DIRECT;
+        else { --J.kv; J.job = JOB_CONN; }
+    } else J.job = JOB_SOURCE;
+}
+__device__ __forceinline__ int job_segment(const PhotonJobs &J) {
+    return J.job == JOB_DIRECT ? 0 : (J.job == JOB_MOVE ? 2 * J.kv - 1 : 2 * J.kv);
+}
+// The end of the job's sweep: how the segment's start depends on what came before it. `add`: this lane adds
+// the start point's share to the gradient.
+template <int FK, class FA>
+__device__ __forceinline__ void job_after(PhotonJobs &J, Lane &L, const KParams &P, const AdjParams &A, const Sweep &w,
+                                          long long sbase, typename FA::Acc &acc, bool add_theta) {
+    const FieldParams &F = P.field;
+    const float4 e0 = traj_get(A, sbase, 0);
+    const float3 p0 = f3(e0.x, e0.y, e0.z);
+    const AdjSeg &g = J.segs[job_segment(J)];
+    if (J.job == JOB_CONN) {
+        // md0 = omega n(pos): the start direction's dependence on n at the vertex
+        const float as = (g.md0[0] * w.Da.x + g.md0[1] * w.Da.y + g.md0[2] * w.Da.z) / w.n0;
+        J.lp = add(J.lp, add(w.Pa, mul(w.gk, as)));
+        J.ld = add(J.ld, J.Ddir);
+        if (add_theta) FA::theta(F, p0, J.s, w.a0 + as, w.b0, acc, A);
+    } else if (J.job == JOB_MOVE) {
+        if (add_theta) FA::theta(F, p0, J.s, w.a0, w.b0, acc, A);
+        J.lp = w.Pa;
+        if (J.kv >= 2) {
+            // the move began with v' = |v| HG(v / |v|) at vertex kv - 1
+            const AdjVertex &c = J.V[J.kv - 1];
+            const int rr_draw = (P.albedo > 0.0f && P.albedo < 1.0f) ? 1 : 0;
+            rng_seek(L, P, c.draws_so + rr_draw);
+            const float u1 = draw(L, P), u2 = draw(L, P);
+            const float gg = P.g;
+            float cosT;
+            if (fabsf(gg) < kEps) cosT = 1.0f - 2.0f * u1;
+            else {
+                const float sq = (1.0f - gg * gg) / (1.0f - gg + 2.0f * gg * u1);
+                cosT = (1.0f + gg * gg - sq * sq) / (2.0f * gg);
+            }
+            const float sinT = sqrtf(fmaxf(0.0f, 1.0f - cosT * cosT));
+            float sP, cP;
+            sincos_red(6.28318548202514648f * u2, sP, cP);
+            J.ld = hg_vjp(f3(c.dir[0], c.dir[1], c.dir[2]), cosT, sinT, cP, sP, w.Da);
+        } else {
+            J.ld = w.Da;
+        }
+    } else {                            // JOB_DIRECT: starts from the source state
+        J.lp = add(J.lp, w.Pa);
+        J.ld = add(J.ld, w.Da);
+        if (add_theta) FA::theta(F, p0, J.s, w.a0, w.b0, acc, A);
+    }
+}
+// The job's sweep, if it has anything to carry.
+__device__ __forceinline__ bool job_setup(PhotonJobs &J, const KParams &P, const AdjParams &A, JobSweep &q,
+                                          unsigned long long &nspl) {
+    q.c = job_segment(J);
+    q.Pa = q.Da = J.Ddir = f3(0.0f, 0.0f, 0.0f);
+    q.a_end = q.T = 0.0f;
+    q.face_end = true;
+    if (J.job == JOB_MOVE) {
+        q.Pa = J.lp; q.Da = J.ld;
+        q.face_end = false;
+        return !(J.lp.x == 0.0f && J.lp.y == 0.0f && J.lp.z == 0.0f && J.ld.x == 0.0f && J.ld.y == 0.0f && J.ld.z == 0.0f);
+    }
+    if (J.job == JOB_CONN ? (J.V[J.kv].hits & 1) : (J.V[0].hits & 2)) {
+        const AdjSeg &g = J.segs[q.c];
+        int ix, iy;
+        float Gt[4];
+        if (g.ok && splat_taps(P, A, f3(g.sp[0], g.sp[1], g.sp[2]), g.spl, g.sdepth, ix, iy, Gt)) {
+            float gr[11];
+            sensor_grad(P, A.X, P.weight, P.sigma_t, P.g, J.job == JOB_CONN, f3(g.mp[0], g.mp[1], g.mp[2]),
+                        f3(g.md[0], g.md[1], g.md[2]), g.mn, g.d2s, f3(g.dir[0], g.dir[1], g.dir[2]),
+                        ix, iy, Gt[0], Gt[1], Gt[2], Gt[3], gr);
+            q.Pa = f3(gr[0], gr[1], gr[2]);
+            q.Da = f3(gr[3], gr[4], gr[5]);
+            q.a_end = gr[6];
+            q.T = gr[7];
+            J.Ddir = f3(gr[8], gr[9], gr[10]);
+            ++nspl;
+            return true;
+        }
+    }
+    return false;
+}
+// the source direction dir0 = n(p0) omega0 (photon.cpp:329)
+template <int FK, class FA>
+__device__ __forceinline__ void job_source(const PhotonJobs &J, const KParams &P, const AdjParams &A, typename FA::Acc &acc,
+                                           bool add_theta) {
+    const FieldParams &F = P.field;
+    if (J.ld.x != 0.0f || J.ld.y != 0.0f || J.ld.z != 0.0f) {
+        const AdjVertex &c = J.V[0];
+        const float3 p0 = f3(c.pos[0], c.pos[1], c.pos[2]);
+        float n0, H[6];
+        float3 g0;
+        FA::eval_h(F, p0, J.s, n0, g0, H);
+        const float as = (c.dir[0] * J.ld.x + c.dir[1] * J.ld.y + c.dir[2] * J.ld.z) / n0;
+        if (add_theta) FA::theta(F, p0, J.s, as, f3(0.0f, 0.0f, 0.0f), acc, A);
+    }
+}
+
+// ---- the spline's sweep: a warp per photon -------------------------------------------------------
+// What a point's step needs from the field -- n, grad n, the Hessian -- follows from the recorded
+// trajectory alone; only the adjoint itself runs from point to point. So a warp evaluates the field at 32
+// points at once, a point a lane, and then carries the adjoint through them, every lane the same, each
+// point's values by shuffles from the lane that has them. A photon swept by one lane takes its chain of
+// evaluations one after the other, and the sweep ends with the longest photon alone in its warp; with 64
+// taps a point to read and as many shares to write that was 106 ms for 40,000 photons on the 64^3 grid,
+// and is 15. Bessel and plane waves have little to evaluate at a point and keep a lane per photon: from
+// about 60,000 photons on a warp each is slower (mode 0, 300,000 photons: 63 against 21 ms).
+// Per warp: the spline weights of 32 points and their cotangents (n, then grad n times the grid's
+// resolution), and per lane the gradient of two taps of the current cell, added up in double and
+// written when the sweep leaves the cell.
+struct SplineShare {
+    float w[32][24];           // wx, wy, wz, dx, dy, dz
+    float4 ab[32];
+};
+struct SplineTaps {
+    int x, y, z;               // the cell
+    double g0, g1;             // taps 2 (lane >> 4) and the next of row lane & 15
+};
+__device__ __forceinline__ void spline_taps_flush(const FieldParams &F, const AdjParams &A, SplineTaps &S, int lane) {
+    if (S.x != INT_MIN && (S.g0 != 0.0 || S.g1 != 0.0)) {
+        const int row = lane & 15, i = 2 * (lane >> 4);
+        double *r = A.grad + (spline_wrap(S.z - 1 + (row >> 2), F.N[2]) * F.N[1] + spline_wrap(S.y - 1 + (row & 3), F.N[1])) * F.N[0];
+        atomicAdd(r + spline_wrap(S.x - 1 + i, F.N[0]), S.g0);
+        atomicAdd(r + spline_wrap(S.x + i, F.N[0]), S.g1);
+    }
+    S.g0 = S.g1 = 0.0;
+}
+// The shares of the lanes with `use`: point p, cotangents (a, b). One warp pass over the points, a lane two
+// of the 64 taps (FieldAdj<FK_SPLINE>::theta's expressions), instead of 64 atomics a point.
+__device__ __forceinline__ void spline_share(const FieldParams &F, const AdjParams &A, SplineShare &M, SplineTaps &S, int lane,
+                                             bool use, float3 p, float a, float3 b) {
+    use = use && !in_gap(F, p);
+    int x = 0, y = 0, z = 0;
+    if (use) {
+        const float t0 = (p.x - F.xmin[0]) * F.xres[0], t1 = (p.y - F.xmin[1]) * F.xres[1], t2 = (p.z - F.xmin[2]) * F.xres[2];
+        float *m = M.w[lane];
+        bspline_weights(t0, m, m + 12);
+        bspline_weights(t1, m + 4, m + 16);
+        bspline_weights(t2, m + 8, m + 20);
+        M.ab[lane] = make_float4(a, b.x * F.xres[0], b.y * F.xres[1], b.z * F.xres[2]);
+        x = int(floorf(t0)); y = int(floorf(t1)); z = int(floorf(t2));
+    }
+    unsigned todo = __ballot_sync(kFull, use);
+    __syncwarp();
+    const int q = lane & 3, c = (lane >> 2) & 3, i = 2 * (lane >> 4);
+    while (todo) {
+        const int l = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        const int lx = __shfl_sync(kFull, x, l), ly = __shfl_sync(kFull, y, l), lz = __shfl_sync(kFull, z, l);
+        if ((lx != S.x) | (ly != S.y) | (lz != S.z)) {
+            spline_taps_flush(F, A, S, lane);
+            S.x = lx; S.y = ly; S.z = lz;
+        }
+        const float *m = M.w[l];
+        const float4 ab = M.ab[l];
+        const float wy = m[4 + q], dy = m[16 + q], wz = m[8 + c], dz = m[20 + c];
+        const float ar = ab.x * wy * wz + ab.z * dy * wz + ab.w * wy * dz;
+        const float br = ab.y * wy * wz;
+        S.g0 += double(ar * m[i] + br * m[12 + i]);
+        S.g1 += double(ar * m[i + 1] + br * m[13 + i]);
+    }
+    __syncwarp();
+}
+
+// Sweeps one segment with the whole warp. 1: the start point is reached (outputs in w); 2: malformed.
+__device__ __forceinline__ int warp_sweep(Sweep &w, const KParams &P, const AdjParams &A, long long base, int len, float3 md_end,
+                                          const JobSweep &q, float s, SplineShare &M, SplineTaps &S, int lane, long long &pts) {
+    typedef FieldAdj<FK_SPLINE> FA;
+    const FieldParams &F = P.field;
+    float c = 0.0f;
+    bool begun = false, junction = false;
+    for (int hi = len - 1; hi >= 0; hi -= 32) {
+        const int idx = hi - lane;
+        const float4 e = idx >= 0 ? traj_get(A, base, idx) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float3 pe = f3(e.x, e.y, e.z);
+        float n = 1.0f, H[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, ta = 0.0f;
+        float3 g = f3(0.0f, 0.0f, 0.0f), tb = g;
+        FA::Cache kc;
+        bool use = false;
+        if (idx >= 0 && (e.w >= 0.0f || idx == len - 1)) {
+            FA::Acc cell;
+            FA::clear(cell);
+            FA::eval_s(F, pe, s, n, g, H, kc, cell);
+        }
+        const int cnt = min(32, hi + 1);
+        int res = 0;
+        for (int l = 0; l < cnt; ++l) {
+            const float ew = __shfl_sync(kFull, e.w, l);
+            if (begun && ew < 0.0f) {               // a reflection between marches
+                junction = true;
+                continue;
+            }
+            const float nl = __shfl_sync(kFull, n, l);
+            const float3 gl = f3(__shfl_sync(kFull, g.x, l), __shfl_sync(kFull, g.y, l), __shfl_sync(kFull, g.z, l));
+            float Hl[6];
+#pragma unroll
+            for (int j = 0; j < 6; ++j) Hl[j] = __shfl_sync(kFull, H[j], l);
+            float3 pl = f3(0.0f, 0.0f, 0.0f);
+            if (!begun || junction) pl = f3(__shfl_sync(kFull, pe.x, l), __shfl_sync(kFull, pe.y, l), __shfl_sync(kFull, pe.z, l));
+            float a;
+            float3 b;
+            if (!begun) {
+                sweep_begin_at(w, P, pl, ew, nl, gl, Hl, md_end, q.Pa, q.Da, q.a_end, q.T, q.face_end, b);
+                a = q.a_end;
+                begun = true;
+            } else {
+                sweep_update(w, P, c, pl, ew, junction, nl, gl, Hl, a, b);
+                ++pts;
+                junction = false;
+                if (ew == 0.0f) { res = 1; break; }
+            }
+            c = ew;
+            if (lane == l) { use = true; ta = a; tb = b; }
+        }
+        spline_share(F, A, M, S, lane, use, pe, ta, tb);
+        if (res) return res;
+    }
+    ++pts;
+    return 2;
+}
+
 // The sweep kernel per field kind; NW bounds the plane-wave count (a plane-wave field of at most two
 // waves runs the NW = 2 instance, whose accumulators take fewer registers); MINB resident blocks.
 template <int FK, int NW> struct FieldAdjSel { typedef FieldAdj<FK> T; };
 template <int NW> struct FieldAdjSel<FK_PLANEWAVE, NW> { typedef FieldAdjPW<NW> T; };
+
+static __global__ void __launch_bounds__(128, 3) adjoint_sweep_warp_kernel(const __grid_constant__ KParams P,
+                                                                          const __grid_constant__ AdjParams A, int round) {
+    typedef FieldAdj<FK_SPLINE> FA;
+    constexpr int FK = FK_SPLINE;
+    const FieldParams &F = P.field;
+    const int lane = threadIdx.x & 31;
+    const long long n_order = (long long)*A.n_order;
+    __shared__ SplineShare s_share[4];                                 // 128-thread blocks
+    SplineShare &M = s_share[threadIdx.x >> 5];
+    Lane L;                                     // Philox draws of the HG rotation
+    L.tab = P.field.btab;
+    L.inst = nullptr;
+    long long pts = 0;
+    unsigned long long nspl = 0, nskip = 0;
+    SplineTaps S;
+    S.x = S.y = S.z = INT_MIN;
+    S.g0 = S.g1 = 0.0;
+    for (;;) {
+        long long q = 0;
+        if (lane == 0) q = (long long)atomicAdd(A.cnt + ADJ_NEXT, 1ull);
+        q = __shfl_sync(kFull, q, 0);
+        if (q >= n_order) break;
+        const long long k = A.order[q];
+        const AdjPhoton r = A.photons[k];
+        if (r.round != round) continue;
+        L.idx = P.first_photon + k;
+        FA::Acc acc;
+        FA::clear(acc);
+        PhotonJobs J;
+        job_photon(J, A, r);
+        while (J.job != JOB_SOURCE) {
+            JobSweep js;
+            const bool run = job_setup(J, P, A, js, nspl);
+            const AdjSeg &g = J.segs[js.c];
+            if (run && g.len >= 2 && (J.job != JOB_MOVE || g.ok)) {
+                Sweep w;
+                const int rr = warp_sweep(w, P, A, g.off, g.len, f3(g.md[0], g.md[1], g.md[2]), js, J.s, M, S, lane, pts);
+                if (rr == 1) job_after<FK, FA>(J, L, P, A, w, g.off, acc, lane == 0);
+                else ++nskip;
+            } else if (run) {
+                ++nskip;
+            }
+            job_next(J);
+        }
+        job_source<FK, FA>(J, P, A, acc, lane == 0);
+    }
+    spline_taps_flush(F, A, S, lane);
+    if (lane == 0) {                            // every lane counted the same
+        atomicAdd(A.cnt + ADJ_POINTS, (unsigned long long)pts);
+        atomicAdd(A.cnt + ADJ_SPLATS, nspl);
+        atomicAdd(A.cnt + ADJ_SKIPPED, nskip);
+    }
+}
 
 template <int FK, int NW, int MINB>
 __global__ void __launch_bounds__(128, MINB) adjoint_sweep_kernel(const __grid_constant__ KParams P,
@@ -1230,15 +1550,14 @@ __global__ void __launch_bounds__(128, MINB) adjoint_sweep_kernel(const __grid_c
     L.inst = nullptr;
     long long pts = 0;
     unsigned long long nspl = 0, nskip = 0;
-    const float albedo = P.albedo;
-    const int rr_draw = (albedo > 0.0f && albedo < 1.0f) ? 1 : 0;
-    const AdjVertex *V = A.pool;
-    const AdjSeg *segs = A.segs;
     const long long n_order = (long long)*A.n_order;
-    int mode = M_DISC, job = 0, kv = 0;
+    int mode = M_DISC;
     bool busy = false;                          // a photon is in progress
-    float s = 0.0f;
-    float3 lp = f3(0.0f, 0.0f, 0.0f), ld = lp, Ddir = lp;
+    PhotonJobs J;
+    J.job = 0; J.kv = 0; J.s = 0.0f;
+    J.lp = J.ld = J.Ddir = f3(0.0f, 0.0f, 0.0f);
+    J.V = A.pool;
+    J.segs = A.segs;
     long long sbase = 0;
     typename FA::Acc acc;
     FA::clear(acc);
@@ -1249,48 +1568,8 @@ __global__ void __launch_bounds__(128, MINB) adjoint_sweep_kernel(const __grid_c
         while (mode == M_DISC) {
             if (after) {
                 after = false;
-                const float4 e0 = traj_get(A, sbase, 0);
-                const float3 p0 = f3(e0.x, e0.y, e0.z);
-                const AdjSeg &g = segs[job == JOB_DIRECT ? 0 : (job == JOB_MOVE ? 2 * kv - 1 : 2 * kv)];
-                if (job == JOB_CONN) {
-                    // md0 = omega n(pos): the start direction's dependence on n at the vertex
-                    const float as = (g.md0[0] * w.Da.x + g.md0[1] * w.Da.y + g.md0[2] * w.Da.z) / w.n0;
-                    lp = add(lp, add(w.Pa, mul(w.gk, as)));
-                    ld = add(ld, Ddir);
-                    FA::theta(F, p0, s, w.a0 + as, w.b0, acc, A);
-                } else if (job == JOB_MOVE) {
-                    FA::theta(F, p0, s, w.a0, w.b0, acc, A);
-                    lp = w.Pa;
-                    if (kv >= 2) {
-                        // the move began with v' = |v| HG(v / |v|) at vertex kv - 1
-                        const AdjVertex &c = V[kv - 1];
-                        rng_seek(L, P, c.draws_so + rr_draw);
-                        const float u1 = draw(L, P), u2 = draw(L, P);
-                        const float gg = P.g;
-                        float cosT;
-                        if (fabsf(gg) < kEps) cosT = 1.0f - 2.0f * u1;
-                        else {
-                            const float sq = (1.0f - gg * gg) / (1.0f - gg + 2.0f * gg * u1);
-                            cosT = (1.0f + gg * gg - sq * sq) / (2.0f * gg);
-                        }
-                        const float sinT = sqrtf(fmaxf(0.0f, 1.0f - cosT * cosT));
-                        float sP, cP;
-                        sincos_red(6.28318548202514648f * u2, sP, cP);
-                        ld = hg_vjp(f3(c.dir[0], c.dir[1], c.dir[2]), cosT, sinT, cP, sP, w.Da);
-                    } else {
-                        ld = w.Da;
-                    }
-                } else {                            // JOB_DIRECT: starts from the source state
-                    lp = add(lp, w.Pa);
-                    ld = add(ld, w.Da);
-                    FA::theta(F, p0, s, w.a0, w.b0, acc, A);
-                }
-                // the next job
-                if (job == JOB_CONN) job = JOB_MOVE;
-                else if (job == JOB_MOVE) {
-                    if (kv == 1) job = JOB_DIRECT;
-                    else { --kv; job = JOB_CONN; }
-                } else job = JOB_SOURCE;
+                job_after<FK, FA>(J, L, P, A, w, sbase, acc, true);
+                job_next(J);
             }
             if (!busy) {
                 const long long q = (long long)atomicAdd(A.cnt + ADJ_NEXT, 1ull);
@@ -1299,73 +1578,30 @@ __global__ void __launch_bounds__(128, MINB) adjoint_sweep_kernel(const __grid_c
                 const AdjPhoton r = A.photons[k];
                 if (r.round != round) continue;
                 L.idx = P.first_photon + k;
-                s = r.s;
-                V = A.pool + r.off;
-                segs = A.segs + 2LL * r.off;
                 FA::clear(acc);
-                FA::begin(acc, L, P, s);
-                lp = f3(0.0f, 0.0f, 0.0f); ld = lp;
-                kv = r.nv - 1;
-                job = kv >= 1 ? JOB_CONN : JOB_DIRECT;
+                FA::begin(acc, L, P, r.s);
+                job_photon(J, A, r);
                 busy = true;
             }
             // set up the current job's sweep, skipping jobs with nothing to carry
-            if (job == JOB_SOURCE) {
-                // dir0 = n(p0) omega0 (photon.cpp:329)
-                if (ld.x != 0.0f || ld.y != 0.0f || ld.z != 0.0f) {
-                    const AdjVertex &c = V[0];
-                    const float3 p0 = f3(c.pos[0], c.pos[1], c.pos[2]);
-                    float n0, H[6];
-                    float3 g0;
-                    FA::eval_h(F, p0, s, n0, g0, H);
-                    const float as = (c.dir[0] * ld.x + c.dir[1] * ld.y + c.dir[2] * ld.z) / n0;
-                    FA::theta(F, p0, s, as, f3(0.0f, 0.0f, 0.0f), acc, A);
-                }
+            if (J.job == JOB_SOURCE) {
+                job_source<FK, FA>(J, P, A, acc, true);
                 FA::flush(acc, F, A);
                 busy = false;
                 continue;
             }
-            const int c = job == JOB_DIRECT ? 0 : (job == JOB_MOVE ? 2 * kv - 1 : 2 * kv);
-            bool run = false, face_end = true;
-            float3 Pa = f3(0.0f, 0.0f, 0.0f), Da = Pa;
-            float a_end = 0.0f, T = 0.0f;
-            Ddir = Pa;
-            if (job == JOB_MOVE) {
-                run = !(lp.x == 0.0f && lp.y == 0.0f && lp.z == 0.0f && ld.x == 0.0f && ld.y == 0.0f && ld.z == 0.0f);
-                Pa = lp; Da = ld;
-                face_end = false;
-            } else if (job == JOB_CONN ? (V[kv].hits & 1) : (V[0].hits & 2)) {
-                const AdjSeg &g = segs[c];
-                int ix, iy;
-                float Gt[4];
-                if (g.ok && splat_taps(P, A, f3(g.sp[0], g.sp[1], g.sp[2]), g.spl, g.sdepth, ix, iy, Gt)) {
-                    float gr[11];
-                    sensor_grad(P, A.X, P.weight, P.sigma_t, P.g, job == JOB_CONN, f3(g.mp[0], g.mp[1], g.mp[2]),
-                                f3(g.md[0], g.md[1], g.md[2]), g.mn, g.d2s, f3(g.dir[0], g.dir[1], g.dir[2]),
-                                ix, iy, Gt[0], Gt[1], Gt[2], Gt[3], gr);
-                    Pa = f3(gr[0], gr[1], gr[2]);
-                    Da = f3(gr[3], gr[4], gr[5]);
-                    a_end = gr[6];
-                    T = gr[7];
-                    Ddir = f3(gr[8], gr[9], gr[10]);
-                    run = true;
-                    ++nspl;
-                }
-            }
-            if (run && segs[c].len >= 2 && (job != JOB_MOVE || segs[c].ok)) {
-                const AdjSeg &g = segs[c];
+            JobSweep q;
+            const bool run = job_setup(J, P, A, q, nspl);
+            if (run && J.segs[q.c].len >= 2 && (J.job != JOB_MOVE || J.segs[q.c].ok)) {
+                const AdjSeg &g = J.segs[q.c];
                 sbase = g.off;
-                sweep_begin<FK, FA>(w, P, A, sbase, g.len, f3(g.md[0], g.md[1], g.md[2]), Pa, Da, a_end, T, face_end, s, acc);
+                sweep_begin<FK, FA>(w, P, A, sbase, g.len, f3(g.md[0], g.md[1], g.md[2]), q.Pa, q.Da, q.a_end, q.T, q.face_end,
+                                    J.s, acc);
                 mode = M_SWEEP;
                 break;
             }
             if (run) ++nskip;
-            // nothing to sweep: the next job, with the adjoint carried as it is
-            if (job == JOB_CONN) job = JOB_MOVE;
-            else if (job == JOB_MOVE) {
-                if (kv == 1) job = JOB_DIRECT;
-                else { --kv; job = JOB_CONN; }
-            } else job = JOB_SOURCE;
+            job_next(J);                        // nothing to sweep: the next job, with the adjoint carried as it is
         }
 
         const unsigned live = __ballot_sync(kFull, mode != M_EXIT);
@@ -1374,17 +1610,13 @@ __global__ void __launch_bounds__(128, MINB) adjoint_sweep_kernel(const __grid_c
         if (__any_sync(kFull, mode == M_SWEEP)) {
             for (;;) {
                 if (mode == M_SWEEP) {
-                    const int rr = sweep_point<FK, FA>(w, P, A, sbase, s, acc);
+                    const int rr = sweep_point<FK, FA>(w, P, A, sbase, J.s, acc);
                     ++pts;
                     if (rr == 1) { mode = M_DISC; after = true; }
                     else if (rr == 2) {
                         mode = M_DISC;
                         ++nskip;
-                        if (job == JOB_CONN) job = JOB_MOVE;
-                        else if (job == JOB_MOVE) {
-                            if (kv == 1) job = JOB_DIRECT;
-                            else { --kv; job = JOB_CONN; }
-                        } else job = JOB_SOURCE;
+                        job_next(J);
                     }
                 }
                 const unsigned idle = __ballot_sync(kFull, mode == M_DISC);
