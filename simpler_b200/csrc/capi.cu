@@ -967,9 +967,8 @@ static int wave_setup(smp_plan *p) {
     p->d_wave = nullptr;
     p->wave_cap = 0;
     auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t b4 = al(n * sizeof(float4)), bi = al(n * sizeof(int4)), bd = al(n * sizeof(double)),
-                 be = al(n * sizeof(EventPart)), bl = al(n * sizeof(int));
-    const size_t bytes = 4 * b4 + bi + bd + be + 4 * bl + 256;
+    const size_t bm = al(6 * n * sizeof(float4)), be = al(n * sizeof(EventPart)), bl = al(n * sizeof(int));
+    const size_t bytes = bm + be + 4 * bl + 256;
     cudaError_t e = cudaMalloc(&p->d_wave, bytes);
     if (e != cudaSuccess) {
         p->d_wave = nullptr;
@@ -979,12 +978,7 @@ static int wave_setup(smp_plan *p) {
     p->wave_cap = n;
     char *b = static_cast<char *>(p->d_wave);
     WaveParams &W = p->wp;
-    W.ma = reinterpret_cast<float4 *>(b); b += b4;
-    W.mb = reinterpret_cast<float4 *>(b); b += b4;
-    W.mc = reinterpret_cast<float4 *>(b); b += b4;
-    W.mdd = reinterpret_cast<float4 *>(b); b += b4;
-    W.mi = reinterpret_cast<int4 *>(b); b += bi;
-    W.mt = reinterpret_cast<double *>(b); b += bd;
+    W.m = reinterpret_cast<float4 *>(b); b += bm;
     W.ev = reinterpret_cast<EventPart *>(b); b += be;
     W.list[0] = reinterpret_cast<int *>(b); b += bl;
     W.list[1] = reinterpret_cast<int *>(b); b += bl;

@@ -8,7 +8,7 @@
 //
 //   wf_march_kernel  -- every slot on the current march list advances up to `chunk` ER steps
 //                       (traceTillBlock, scene.cpp:385-425). Only the march state is loaded
-//                       (88 bytes, structure-of-arrays, coalesced), so the kernel runs at a small
+//                       (one 96-byte record), so the kernel runs at a small
 //                       register count and high occupancy with no event code in its instruction
 //                       stream. Slots whose march ended go to the event queue; the rest go
 //                       straight to the next march list.
@@ -72,13 +72,14 @@ __device__ __forceinline__ void ev_store(EventPart *dst, const EventPart &E) {
 }
 
 struct WaveParams {
-    // march state, structure of arrays
-    float4 *ma;        // mp.xyz, mn
-    float4 *mb;        // md.xyz, cur
-    float4 *mc;        // mg.xyz, dist_acc
-    float4 *mdd;       // dlimit, s, mtotf, instance index (bits; batched sweep)
-    int4 *mi;          // steps, end, prec, stop
-    double *mt;        // mtot (FP64 path-length form only)
+    // March state, one record of six 16-byte pieces per slot: (mp, mn), (md, cur), (mg, dist_acc),
+    // (dlimit, s, mtotf, instance index bits), (steps, end, prec, stop), mtot (FP64 path-length form
+    // only). The lists hold slots in no order, so a piece on its own is half a 32-byte sector read for
+    // nothing; a record's 96 bytes are three whole ones.
+    float4 *m;
+    __device__ __forceinline__ float4 *rec(int slot) const { return m + 6 * size_t(slot); }
+    __device__ __forceinline__ int4 *rec_i(int slot) const { return reinterpret_cast<int4 *>(rec(slot) + 4); }
+    __device__ __forceinline__ double *rec_d(int slot) const { return reinterpret_cast<double *>(rec(slot) + 5); }
     EventPart *ev;
     int *list[2];      // march lists, by iteration parity
     int *queue[2];     // event queues, by iteration parity
@@ -157,8 +158,8 @@ __device__ __forceinline__ int brick_slot(const WaveParams &W, int par, unsigned
 }
 
 __device__ __forceinline__ void wf_load_march(const WaveParams &W, const KParams &P, int slot, MarchState &M) {
-    const float4 a = W.ma[slot], b = W.mb[slot], c = W.mc[slot], d = W.mdd[slot];
-    const int4 e = W.mi[slot];
+    const float4 a = W.rec(slot)[0], b = W.rec(slot)[1], c = W.rec(slot)[2], d = W.rec(slot)[3];
+    const int4 e = *W.rec_i(slot);
     M.mp = f3(a.x, a.y, a.z); M.mn = a.w;
     M.md = f3(b.x, b.y, b.z); M.cur = b.w;
     M.mg = f3(c.x, c.y, c.z); M.dist_acc = c.w;
@@ -167,17 +168,17 @@ __device__ __forceinline__ void wf_load_march(const WaveParams &W, const KParams
     M.inst = P.n_inst ? P.insts + __float_as_int(d.w) : nullptr;
     M.hh = 0.5f * M.cur;
     M.cur_d = double(M.cur);
-    M.mtot = P.fp64 ? W.mt[slot] : 0.0;
+    M.mtot = P.fp64 ? *W.rec_d(slot) : 0.0;
 }
 
 template <class S>
 __device__ __forceinline__ void wf_store_march(const WaveParams &W, const KParams &P, int slot, const S &M) {
-    W.ma[slot] = make_float4(M.mp.x, M.mp.y, M.mp.z, M.mn);
-    W.mb[slot] = make_float4(M.md.x, M.md.y, M.md.z, M.cur);
-    W.mc[slot] = make_float4(M.mg.x, M.mg.y, M.mg.z, M.dist_acc);
-    W.mdd[slot] = make_float4(M.dlimit, M.s, M.mtotf, __int_as_float(P.n_inst ? int(M.inst - P.insts) : 0));
-    W.mi[slot] = make_int4(M.steps, M.end, M.prec, M.stop);
-    if (P.fp64) W.mt[slot] = M.mtot;
+    W.rec(slot)[0] = make_float4(M.mp.x, M.mp.y, M.mp.z, M.mn);
+    W.rec(slot)[1] = make_float4(M.md.x, M.md.y, M.md.z, M.cur);
+    W.rec(slot)[2] = make_float4(M.mg.x, M.mg.y, M.mg.z, M.dist_acc);
+    W.rec(slot)[3] = make_float4(M.dlimit, M.s, M.mtotf, __int_as_float(P.n_inst ? int(M.inst - P.insts) : 0));
+    *W.rec_i(slot) = make_int4(M.steps, M.end, M.prec, M.stop);
+    if (P.fp64) *W.rec_d(slot) = M.mtot;
 }
 
 __device__ __forceinline__ void wf_load_lane(const WaveParams &W, const KParams &P, int slot, Lane &L) {
@@ -280,8 +281,8 @@ wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveP
         if (valid) {
             slot = two_class_at(W.list[cur], n0, W.n_slots, i);
             MarchStateT<typename MarchTable<REP>::T> M;
-            const float4 a = W.ma[slot], b = W.mb[slot], c = W.mc[slot], d = W.mdd[slot];
-            const int4 e = W.mi[slot];
+            const float4 a = W.rec(slot)[0], b = W.rec(slot)[1], c = W.rec(slot)[2], d = W.rec(slot)[3];
+            const int4 e = *W.rec_i(slot);
             M.mp = f3(a.x, a.y, a.z); M.mn = a.w;
             M.md = f3(b.x, b.y, b.z); M.cur = b.w;
             M.mg = f3(c.x, c.y, c.z); M.dist_acc = c.w;
@@ -289,7 +290,7 @@ wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveP
             M.steps = e.x; M.end = 0; M.prec = e.z; M.stop = e.w;   // a marching slot has no end code
             M.hh = 0.5f * M.cur;
             M.cur_d = double(M.cur);
-            M.mtot = F64 ? W.mt[slot] : 0.0;
+            M.mtot = F64 ? *W.rec_d(slot) : 0.0;
             M.tab = tab;
             if constexpr (FK == FK_BATCH) {
                 M.inst = P.insts + __float_as_int(d.w);
@@ -308,12 +309,12 @@ wf_march_kernel(const __grid_constant__ KParams P, const __grid_constant__ WaveP
                 }
             }
             done += unsigned(M.steps - steps0);
-            W.ma[slot] = make_float4(M.mp.x, M.mp.y, M.mp.z, M.mn);
-            W.mb[slot] = make_float4(M.md.x, M.md.y, M.md.z, M.cur);
-            W.mc[slot] = make_float4(M.mg.x, M.mg.y, M.mg.z, M.dist_acc);
-            if (F64) W.mt[slot] = M.mtot;
-            else W.mdd[slot] = make_float4(M.dlimit, M.s, M.mtotf, d.w);
-            W.mi[slot] = make_int4(M.steps, M.end, M.prec, M.stop);
+            W.rec(slot)[0] = make_float4(M.mp.x, M.mp.y, M.mp.z, M.mn);
+            W.rec(slot)[1] = make_float4(M.md.x, M.md.y, M.md.z, M.cur);
+            W.rec(slot)[2] = make_float4(M.mg.x, M.mg.y, M.mg.z, M.dist_acc);
+            if (F64) *W.rec_d(slot) = M.mtot;
+            else W.rec(slot)[3] = make_float4(M.dlimit, M.s, M.mtotf, d.w);
+            *W.rec_i(slot) = make_int4(M.steps, M.end, M.prec, M.stop);
         }
         const unsigned em = __ballot_sync(kFull, valid && ended);
         const unsigned cm = __ballot_sync(kFull, valid && !ended);
@@ -438,8 +439,8 @@ wf_march_spline_kernel(const __grid_constant__ KParams P, const __grid_constant_
         if (valid) {
             slot = W.blist[cur][size_t(b) * size_t(W.bstride) + i];
             MarchState M;
-            const float4 a = W.ma[slot], bb = W.mb[slot], c = W.mc[slot], d = W.mdd[slot];
-            const int4 e = W.mi[slot];
+            const float4 a = W.rec(slot)[0], bb = W.rec(slot)[1], c = W.rec(slot)[2], d = W.rec(slot)[3];
+            const int4 e = *W.rec_i(slot);
             M.mp = f3(a.x, a.y, a.z); M.mn = a.w;
             M.md = f3(bb.x, bb.y, bb.z); M.cur = bb.w;
             M.mg = f3(c.x, c.y, c.z); M.dist_acc = c.w;
@@ -447,7 +448,7 @@ wf_march_spline_kernel(const __grid_constant__ KParams P, const __grid_constant_
             M.steps = e.x; M.end = 0; M.prec = e.z; M.stop = e.w;   // a marching slot has no end code
             M.hh = 0.5f * M.cur;
             M.cur_d = double(M.cur);
-            M.mtot = F64 ? W.mt[slot] : 0.0;
+            M.mtot = F64 ? *W.rec_d(slot) : 0.0;
             M.tab = brick;
             M.inst = nullptr;
             const int steps0 = M.steps;
@@ -456,12 +457,12 @@ wf_march_spline_kernel(const __grid_constant__ KParams P, const __grid_constant_
                 if (march_step<FK_SPLINE, F64>(M, P, C) || march_step<FK_SPLINE, F64>(M, P, C)) { ended = true; break; }
             }
             done += unsigned(M.steps - steps0);
-            W.ma[slot] = make_float4(M.mp.x, M.mp.y, M.mp.z, M.mn);
-            W.mb[slot] = make_float4(M.md.x, M.md.y, M.md.z, M.cur);
-            W.mc[slot] = make_float4(M.mg.x, M.mg.y, M.mg.z, M.dist_acc);
-            if (F64) W.mt[slot] = M.mtot;
-            else W.mdd[slot] = make_float4(M.dlimit, M.s, M.mtotf, d.w);
-            W.mi[slot] = make_int4(M.steps, M.end, M.prec, M.stop);
+            W.rec(slot)[0] = make_float4(M.mp.x, M.mp.y, M.mp.z, M.mn);
+            W.rec(slot)[1] = make_float4(M.md.x, M.md.y, M.md.z, M.cur);
+            W.rec(slot)[2] = make_float4(M.mg.x, M.mg.y, M.mg.z, M.dist_acc);
+            if (F64) *W.rec_d(slot) = M.mtot;
+            else W.rec(slot)[3] = make_float4(M.dlimit, M.s, M.mtotf, d.w);
+            *W.rec_i(slot) = make_int4(M.steps, M.end, M.prec, M.stop);
             if (!ended) key = spline_brick_of(P.field, W, M.mp);
         }
         const unsigned em = __ballot_sync(kFull, valid && ended);
