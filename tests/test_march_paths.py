@@ -1,0 +1,213 @@
+"""The ways a photon can be marched -- the pool's march kernel with one or several copies of the Bessel
+table, untested windows, a spline cell kept in registers, the whole warp on a lone spline photon, small
+renders as one launch -- against the plain kernel, one thread per photon with every step tested. All
+run the same arithmetic in the same order, so the photon records have to be the same bytes; FP64 films
+differ by the order of their sums alone (2^-53 a term, 1e-12 of the film's sum)."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+import simpler_b200 as sb
+from simpler_b200 import _lib as L
+
+MIXED = dict(precision_mode=L.PREC_MIXED)
+
+
+def spline(n, box=None, **kw):
+    s = sb.config_spline(n, 4)
+    if box:
+        s.grid_min, s.grid_max = box
+    for k, v in kw.items():
+        setattr(s, k, v)
+    return s
+
+
+SETUPS = {
+    "mode0": lambda: sb.config_plain_small(mode=0, seed=1),
+    "mode1_mixed": lambda: sb.config_plain_small(mode=1, seed=2, f_u=1.9e6, **MIXED),
+    "mode2": lambda: sb.config_plain_small(mode=2, seed=3),
+    "mode5": lambda: sb.config_plain_small(mode=5, seed=4),
+    "gaps": lambda: sb.config_plain_small(mode=2, emitter_gap=2e-3, sensor_gap=1.3e-3, seed=5),
+    "off_centre_box": lambda: sb.config_plain_small(mode=1, medium_l=(-4e-3, -3.3e-3, -6e-3),
+                                                    medium_r=(5e-3, 4.1e-3, 2.1e-3), seed=6),
+    "long_step": lambda: sb.config_plain_small(mode=1, er_stepsize=3e-4, seed=7),
+    "short_step": lambda: sb.config_plain_small(mode=0, er_stepsize=1e-6, sigma_t=4000.0, seed=8),
+    "no_refinement": lambda: sb.config_plain_small(mode=0, precision=0, seed=9),
+    "no_field": lambda: sb.config_plain_small(mode=0, n_max=0.0, n_clip=0.0, seed=10),
+    "strong_field": lambda: sb.config_plain_small(mode=1, n_max=0.2, n_clip=0.1, seed=11),     # no window bound
+    "wave1": lambda: sb.config_planewave(wave_amp=(1e-3,), wave_k=((0.0, 4000.0, 0.0),), wave_phase=(0.3,), seed=12),
+    "wave8": lambda: sb.config_planewave(wave_amp=(2e-4,) * 8, wave_phase=(0.1,) * 8, seed=13, **MIXED,
+                                         wave_k=tuple((100.0 * i, 3000.0, -500.0 * i) for i in range(8))),
+    "spline64": lambda: spline(64, seed=14),
+    "spline13_mixed": lambda: spline(13, seed=15, **MIXED),
+    "spline_gap": lambda: spline(24, seed=16, emitter_gap=1e-3),
+    # a grid that ends inside the box: points one cell off it, and further off (taps one by one)
+    "spline_inside": lambda: spline(17, box=((-4e-3, -5e-3, -3e-3), (3e-3, 4.9e-3, 5e-3)), seed=17),
+}
+
+
+def records(setup, n):
+    recs, _ = sb.trace_photons(setup, 0, n, n, with_image=False)
+    return sb.records_to_arrays(recs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(SETUPS))
+def test_photons_are_the_plain_kernels(name, monkeypatch):
+    s = SETUPS[name]()
+    n = 300 if name in ("short_step", "spline_inside") else 2500
+    ref = records(dataclasses.replace(s, kernel=L.KERNEL_PLAIN), n)
+    assert (ref["er_steps"] > 0).any()
+    for direct in ("1000000", "0"):                       # one launch; the pool and its tail
+        monkeypatch.setenv("SMP_WF_DIRECT", direct)
+        got = records(s, n)
+        assert got.tobytes() == ref.tobytes(), (name, direct, int((got["er_steps"] != ref["er_steps"]).sum()))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 33, 593, 2369, 40000, 40001])
+def test_small_renders_around_the_one_launch_limit(n):
+    """1 photon, part of a warp, more photons than warps, and both sides of the line between the one
+    launch and the pool."""
+    s = sb.config_plain_small(mode=1, seed=20, spatial_x=33, spatial_y=17, path_length_bins=5, sensor_march_max=0.05, **MIXED)
+    film, st = sb.render(s, n)
+    ref, rst = sb.render(dataclasses.replace(s, kernel=L.KERNEL_PLAIN), n)
+    assert (st.photons, st.er_steps, st.splats) == (rst.photons, rst.er_steps, rst.splats) and st.photons == n
+    assert st.launches == 1 if n <= 40000 else st.launches > 1
+    assert np.abs(film - ref).sum() <= 1e-12 * np.abs(ref).sum()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("block", [128, 256])
+@pytest.mark.parametrize("f_u", [0.3e6, 1.0e6, 1.3e6, 2.4e6, 4.0e6])
+def test_table_copies(f_u, block, monkeypatch):
+    """k r up to 10 .. 120: four, two and one copies of the table in either block size."""
+    monkeypatch.setenv("SMP_WF_BLOCK", str(block))
+    monkeypatch.setenv("SMP_WF_DIRECT", "0")
+    s = sb.config_plain_small(mode=1, f_u=f_u, seed=30, sensor_march_max=0.05)
+    got, ref = records(s, 20000), records(dataclasses.replace(s, kernel=L.KERNEL_PLAIN), 20000)
+    assert got.tobytes() == ref.tobytes()
+
+
+@pytest.mark.gpu
+def test_batched_windows(monkeypatch):
+    """A sweep's small films by the one launch and by the pool, orders 0-2, the film's order of sums apart."""
+    setup, insts = sb.config_batch_sweep(n_inst=7, seed=5, scale=3e-3, **MIXED)
+    for i, x in enumerate(insts):
+        x["er_stepsize"] = (1e-5, 4e-5, 1.6e-4)[i % 3]
+    assert {x["mode"] for x in insts} == {0, 1, 2} and sum(x["n_photons"] for x in insts) > 7
+    out = []
+    for direct in ("1000000", "0"):
+        monkeypatch.setenv("SMP_WF_DIRECT", direct)
+        monkeypatch.setenv("SMP_TUNE", "0")
+        films, st = sb.render_batch(setup, insts)
+        out.append((films, st.photons, st.er_steps, st.splats))
+    assert out[0][1:] == out[1][1:]
+    assert np.abs(out[0][0] - out[1][0]).sum() <= 1e-12 * np.abs(out[0][0]).sum()
+
+
+def splat_sum(s, rec):
+    """The film of the records' splats (addEnergyToImage's bilinear split, scene.cpp:782-829), in the
+    renderer's own float arithmetic up to the taps' values, added in double."""
+    f = np.float32
+    sc = s.scene_desc()
+    Z, Y, X = s.film_shape()
+    film = np.zeros((Z, Y, X))
+    o, plane = np.array(sc.view_origin[:], f), np.array(sc.view_plane[:], f)
+    lo, hi = np.float64(f(s.path_length_min)), np.float64(f(s.path_length_max))
+    for k in range(rec["splats"].shape[1]):
+        sp = rec["splats"][rec["n_splats"] > k, k]
+        p, pl, val = sp["p"].astype(f), sp["pathlength"], sp["value"].astype(f)
+        sp_ok = (pl > lo) & (pl < hi)
+        p, pl, val = p[sp_ok], pl[sp_ok], val[sp_ok]
+        x = ((-p[:, 1] - o[1]) / plane[0] + f(0.5)) * f(X)      # horizontal -y; vertical dir x horizontal = z
+        y = ((p[:, 2] - o[2]) / plane[1] + f(0.5)) * f(Y)
+        iz = np.floor((pl - lo) / (hi - lo) * Z).astype(int)
+        ix, iy = np.floor(x), np.floor(y)
+        fx, fy = x - ix, y - iy
+        ix, iy = ix.astype(int), iy.astype(int)
+        one = f(1.0)
+        for dx, dy, w in ((0, 0, val * (one - fx) * (one - fy)), (1, 0, val * fx * (one - fy)),
+                          (0, 1, val * (one - fx) * fy), (1, 1, val * fx * fy)):
+            m = (ix + dx >= 0) & (ix + dx < X) & (iy + dy >= 0) & (iy + dy < Y) & (iz >= 0) & (iz < Z)
+            np.add.at(film, (iz[m], iy[m] + dy, ix[m] + dx), w[m].astype(np.float64))
+    return film
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("x,y,z", [(1, 1, 1), (2, 3, 1), (5, 2, 7), (64, 64, 16), (301, 7, 3)])
+def test_splats_that_share_pixels(x, y, z):
+    """Whole warps in one pixel (a 1 x 1 film) to hardly any two lanes in one, base pixels at -1 included:
+    the film is the sum of the records' splats. Both sides add the same float taps in double; the vertical
+    axis (0, 0, 1) and horizontal (0, -1, 0) make the projections exact."""
+    s = sb.config_plain_small(mode=0, seed=40, spatial_x=x, spatial_y=y, path_length_bins=z, sensor_march_max=0.04,
+                              max_depth=4, **MIXED)
+    recs, film = sb.trace_photons(s, 0, 4000, 4000)
+    rec = sb.records_to_arrays(recs)
+    assert rec["n_splats"].max() <= rec["splats"].shape[1]
+    ref = splat_sum(s, rec)
+    assert ref.sum() > 0
+    assert np.abs(film - ref).sum() <= 1e-12 * np.abs(ref).sum()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nt,nz,kw", [(2, 2, {}), (3, 5, {}), (4, 1, {"trans_z_sources": 2}), (5, 7, {"n_coeff": 3}),
+                                      (100, 3, {"active1": False}), (101, 4, {"active2": False, "phase2": 1.0}),
+                                      (440, 2, {}), (441, 2, {})])
+def test_source_values_are_the_field_evaluations(nt, nz, kw):
+    """Rows shorter than, equal to and longer than the four places of a 16-byte load, the longest that
+    shared memory holds and one more (which takes the probe), 1 to 300 points, points in the gap."""
+    import ctypes as C
+    s = sb.config_sources(theta_sources=nt, **{"trans_z_sources": nz, **kw}, emitter_gap=1e-3, sensor_gap=5e-4)
+    fd = s.field_desc()
+    for n in (1, 127, 128, 300):
+        pts = np.ascontiguousarray(np.random.default_rng(n).uniform(-5e-3, 5e-3, (n, 3)))
+        want, _ = sb.field_eval(s, 0.0, pts)
+        got = np.zeros(n)
+        L.check(sb.load().smp_field_values(C.byref(fd), 0.0, n, C.c_void_p(pts.ctypes.data), C.c_void_p(got.ctypes.data)))
+        assert np.array_equal(got, want)
+
+
+def test_source_values_rejects_bad_arguments():
+    lib = sb.load()
+    assert lib.smp_field_values(None, 0.0, 1, None, None) == L.SMP_ERR_BAD_ARG
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("step", [1e-5, 2.9e-4, 3.4e-4])
+def test_spline_gradient_around_the_sweeps_chunk(step):
+    """The spline's sweep takes 32 points at a time: segments of about 1000, 35 and 30 points and their refined
+    ends. Direct light, FP64 film, differenced along the gradient itself by a step that changes the
+    objective J by 1e-4: J's own rounding is 2e-6 of a photon's value (a position's float rounding against
+    a 0.16 mm pixel), 1.4e-8 of J over 20,000 photons, and the central difference's cubic term is below
+    1e-3 of the change at a field change of a few per cent; 1e-2 is ten times their sum."""
+    from test_adjoint import smooth_weights
+    s = sb.config_spline(16, 4, albedo=0.0, er_stepsize=step, spatial_x=64, spatial_y=64, path_length_bins=4, **MIXED)
+    G = smooth_weights(s)
+    n_ph = 20000
+    grad, st = sb.adjoint(s, n_ph, G)
+    assert st.dropped == st.skipped == st.aborted == st.replay_mismatch == 0 and st.photons == n_ph
+    J = float((sb.render(s, n_ph)[0] * G).sum())
+    d = (grad * (0.5e-4 * abs(J) / float(grad @ grad))).reshape(s.grid_coeff.shape)
+    up, dn = ((s.grid_coeff + k * d).astype(np.float32) for k in (1.0, -1.0))
+    fu, fd = (sb.render(dataclasses.replace(s, grid_coeff=c), n_ph)[0] for c in (up, dn))
+    quotient = float(((fu - fd) * G).sum())
+    predicted = float(grad @ (up.astype(np.float64) - dn.astype(np.float64)).ravel())
+    assert abs(predicted - quotient) <= 1e-2 * abs(quotient), (predicted, quotient)
+
+
+@pytest.mark.parametrize("shape", [(2, 2, 2), (3, 5, 4), (17, 2, 9), (40, 33, 3)])
+def test_prefilter_shapes_against_the_oracle(shape):
+    """Two samples on an axis and unequal axes, 2e-6 as in the cubic grid's own test (values near 1.3333)."""
+    import ctypes as C
+
+    import oracle_bridge as ob
+    n = np.array(shape[::-1], np.int32)
+    s = (1.3333 + 1e-3 * np.random.default_rng(2).standard_normal(shape)).astype(np.float32)
+    got = np.zeros_like(s)
+    p = lambda a: C.c_void_p(a.ctypes.data)                # noqa: E731
+    sb._lib.check(sb.load().smp_spline_prefilter(p(s), p(n), p(got)))
+    ref, s64 = np.zeros(s.size), s.astype(np.float64)
+    ob.oracle().orc_spline_prefilter3d(p(s64), p(n), 32, p(ref))
+    assert np.allclose(got.reshape(-1), ref, rtol=0, atol=2e-6)
