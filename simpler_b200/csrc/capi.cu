@@ -540,9 +540,11 @@ struct smp_plan {
     int march_copies = 1;       // copies of the Bessel table in the march kernel's shared memory
     bool tuned = false;         // the schedule came from smp_plan_tune
     size_t wave_cap = 0;        // slots the pool allocation holds
-    long long direct_max = 40000;   // renders of at most this many photons are one launch of the tail
-                                    // kernel, with no pool (SMP_WF_DIRECT)
-    long long finish_max = 1LL << 30;
+    // Renders of at most this many photons are one launch of the tail kernel, with no pool
+    // (SMP_WF_DIRECT). 9001 spline photons take 54 ms either way and 120,000 Bessel photons 18 and 20
+    // ms, so the line lies where the launches saved (66 and more) and the pool's 150 MB still count.
+    long long direct_max = 40000;
+    long long pool_traces = 0;      // traces that took the pool since the last clear
     int wave_batch = 16;        // march/event launch pairs between live-slot checks
     int wave_split = 1;         // march lists and event queues by march class (WaveParams.split)
     void *d_wave = nullptr;
@@ -779,7 +781,6 @@ int smp_plan_create(const smp_scene_desc *scene, const smp_medium_desc *medium, 
     }
     if (const char *c = std::getenv("SMP_WF_BATCH")) p->wave_batch = std::max(1, std::min(256, std::atoi(c)));
     if (const char *c = std::getenv("SMP_WF_DIRECT")) p->direct_max = std::atoll(c);
-    if (const char *c = std::getenv("SMP_WF_FINISH")) p->finish_max = std::atoll(c);
     if (const char *c = std::getenv("SMP_WF_SPLIT")) p->wave_split = std::atoi(c) != 0;
     p->scene = *scene;
     p->medium = *medium;
@@ -899,6 +900,7 @@ int smp_plan_clear(smp_plan *plan, void *stream) {
     plan->march_ev_used = 0;
     plan->graph_march_launches = 0;
     plan->n_launched = 0;
+    plan->pool_traces = 0;
     std::memset(&plan->stats, 0, sizeof(plan->stats));
     return SMP_OK;
 }
@@ -1054,13 +1056,14 @@ static int wave_run(smp_plan *p, const KParams &k, cudaStream_t s) {
     }
     int rc = wave_setup(p);
     if (rc) return rc;
+    p->pool_traces += 1;
     WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, p->wp.nb > 0, p->march_copies), fe = wf_event_fn(p->fk),
            ff = wf_finish_fn(p->fk);
     WaveParams W = p->wp;
     const int mb = p->march_block;
     if (W.nb > 0) SMP_CUDA(cudaMemsetAsync(W.bcnt[0], 0, 2 * size_t(W.nb) * sizeof(unsigned), s));
     // once the live slots fit in one persistent grid, the finisher runs them to the end
-    const unsigned finish_at = unsigned(std::min<long long>((long long)p->grid_finish * kBlock, p->finish_max));
+    const unsigned finish_at = unsigned(p->grid_finish) * unsigned(kBlock);
     SMP_CUDA(cudaMemsetAsync(W.cnt, 0, 8 * sizeof(unsigned), s));
     fe<<<p->grid_event, kBlock, 0, s>>>(k, W, -1);
     SMP_CUDA(cudaGetLastError());
@@ -1239,7 +1242,8 @@ static int collect_stats(smp_plan *plan) {
         SMP_CUDA(cudaEventElapsedTime(&ms, plan->march_ev[i], plan->march_ev[i + 1]));
         march_ms += ms;
     }
-    const bool one_kernel = plan->kernel != SMP_KERNEL_POOL;      // march and events in one kernel
+    // march and events in one kernel
+    const bool one_kernel = plan->kernel != SMP_KERNEL_POOL || (plan->n_launched > 0 && plan->pool_traces == 0);
     plan->stats.march_ms = one_kernel ? ms_total : march_ms;
     plan->stats.march_steps = one_kernel ? (int64_t)c[CNT_STEPS] : (int64_t)c[CNT_MARCH_STEPS];
     plan->stats.launches = plan->n_launched;
@@ -1409,6 +1413,13 @@ static int plan_tune(smp_plan *plan, int64_t n_sample, int64_t n_grow, smp_tunin
             return smp_plan_clear(plan, nullptr);
         }
     }
+    // the trials time the pool, whatever the sample
+    struct PoolOnly {
+        smp_plan *p;
+        long long keep;
+        explicit PoolOnly(smp_plan *q) : p(q), keep(q->direct_max) { q->direct_max = 0; }
+        ~PoolOnly() { p->direct_max = keep; }
+    } pool_only(plan);
     // n_inst > 0 (a batched sweep): each instance carries its own weight, the argument is unused
     const int64_t weight = n_sample;
     static const int kSlots[4] = {8, 6, 4, 2};      // largest first: the pool is allocated once
