@@ -540,10 +540,13 @@ struct smp_plan {
     int march_copies = 1;       // copies of the Bessel table in the march kernel's shared memory
     bool tuned = false;         // the schedule came from smp_plan_tune
     size_t wave_cap = 0;        // slots the pool allocation holds
-    // Renders of at most this many photons are one launch of the tail kernel, with no pool
-    // (SMP_WF_DIRECT). 9001 spline photons take 54 ms either way and 120,000 Bessel photons 18 and 20
-    // ms, so the line lies where the launches saved (66 and more) and the pool's 150 MB still count.
-    long long direct_max = 40000;
+    // Renders of at most two photons per lane of the tail kernel's grid (one for the spline) are one launch
+    // of that kernel, with no pool (SMP_WF_DIRECT: of at most that many photons; -1: this rule). Resident plans
+    // of Bessel and plane-wave fields take the same time either way up to 2.6 photons a lane (60,000 to
+    // 200,000 photons: 13.4 to 19.8 against 13.3 to 18.8 ms, mode 0), and a one-shot render is spared
+    // the pool's 150 MB and a hundred launches (120,000 photons 30 to 25 ms). The spline's pool pays
+    // sooner: 9,000 photons take 54 ms either way, 200,000 213 against 160.
+    long long direct_max = -1;
     long long pool_traces = 0;      // traces that took the pool since the last clear
     int wave_batch = 16;        // march/event launch pairs between live-slot checks
     int wave_split = 1;         // march lists and event queues by march class (WaveParams.split)
@@ -952,7 +955,7 @@ static int wave_setup(smp_plan *p) {
     p->march_smem = bricks ? size_t(kBrickSmemBytes) : p->smem_bytes * size_t(p->march_copies);
     int sms = 0, pm = 0, pe = 0;
     int rc = allow_dynamic_smem(reinterpret_cast<const void *>(fm), p->march_smem);
-    if (!rc) rc = finish_setup(p);
+    if (!rc) rc = finish_setup(p);                  // wave_run's own callers have not
     if (rc) return rc;
     SMP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, p->device));
     SMP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pm, fm, p->march_block, p->march_smem));
@@ -1042,11 +1045,13 @@ static unsigned long long live_of(unsigned long long word) {
 // wave_batch pairs until no slot is live. The live count after each batch is read back while the
 // next batch is already queued, so the device does not idle during the check.
 static int wave_run(smp_plan *p, const KParams &k, cudaStream_t s) {
-    if (!p->bricks && k.n_photons <= p->direct_max) {
-        int rc = finish_setup(p);
-        if (rc) return rc;
+    int rc = finish_setup(p);
+    if (rc) return rc;
+    const long long lanes = (long long)p->grid_finish * kBlock;
+    const long long direct = p->direct_max >= 0 ? p->direct_max : (p->fk == FK_SPLINE ? 1 : 2) * lanes;
+    if (!p->bricks && k.n_photons <= direct) {
         KParams kd = k;
-        kd.fetch_from = std::min<long long>(k.n_photons, (long long)p->grid_finish * kBlock);
+        kd.fetch_from = std::min<long long>(k.n_photons, lanes);
         WaveParams W;
         std::memset(&W, 0, sizeof(W));
         wf_finish_fn(p->fk)<<<p->grid_finish, kBlock, p->smem_bytes, s>>>(kd, W, -1);
@@ -1054,7 +1059,7 @@ static int wave_run(smp_plan *p, const KParams &k, cudaStream_t s) {
         p->n_launched += 1;
         return SMP_OK;
     }
-    int rc = wave_setup(p);
+    rc = wave_setup(p);
     if (rc) return rc;
     p->pool_traces += 1;
     WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, p->wp.nb > 0, p->march_copies), fe = wf_event_fn(p->fk),
