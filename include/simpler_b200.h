@@ -178,10 +178,9 @@ typedef struct smp_render_opts {
     int32_t  kernel;              /* smp_kernel: which kernel traces the photons (0 = the default)   */
     /* Spline fields on the slot pool: 1 stages the coefficient grid in bricks of 16^3 cells in
        shared memory with the Tensor Memory Accelerator and bins the march lists by brick; 0 (the
-       default) reads the taps through the L1 cache. Both give the same photons. The march is bound
-       by the L1/shared-memory data path either way (16 random 16-byte gathers per evaluation), and
-       the staged bricks' shared-memory gathers conflict in banks and halve the resident warps, so the
-       default is measurably faster on B200. */
+       default) keeps the taps of a march's current cell in registers, read once per cell. Both give
+       the same photons. The bricks' shared-memory gathers, sixteen a step, conflict in banks and halve
+       the resident warps, so the default is measurably faster on B200 (5 times in the march). */
     int32_t  spline_bricks;
 } smp_render_opts;
 
@@ -189,7 +188,8 @@ typedef struct smp_render_opts {
    photons are identical; they differ in scheduling. */
 typedef enum smp_kernel {
     SMP_KERNEL_POOL       = 0,    /* the default: march and event kernels alternating over a
-                                     resident pool of photon slots, with a persistent tail kernel  */
+                                     resident pool of photon slots, with a persistent tail kernel;
+                                     renders of few photons are one launch of the tail kernel      */
     SMP_KERNEL_PERSISTENT = 1,    /* one persistent launch; each lane runs its photons to the end
                                      and takes the next index from a global counter                */
     SMP_KERNEL_PLAIN      = 2     /* one thread per photon in one launch, no regeneration: the

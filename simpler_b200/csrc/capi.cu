@@ -163,8 +163,8 @@ static void source_centres(const smp_field_desc &f, std::vector<float4> &out) {
     }
 }
 
-// The offsets as x-tap quads (FieldParams.coeff4): entry row * N0 + x holds the offsets at the
-// mirrored x - 1, x, x + 1, x + 2 of that row, the four taps of a point with floor(t_x) = x.
+// The offsets as x-tap quads (FieldParams.coeff4): entry row * (N0 + 2) + 1 + x, x = -1 .. N0, holds the
+// offsets at the mirrored x - 1, x, x + 1, x + 2 of that row, the four taps of a point with floor(t_x) = x.
 static int spline_mirror(int i, int n) {
     int m = 2 * n - 2, w = i % m;
     if (w < 0) w += m;
@@ -939,17 +939,19 @@ static int finish_setup(smp_plan *p) {
     return SMP_OK;
 }
 
+// Copies of the Bessel table (dev_field.cuh RepTable) as long as the SM's resident blocks hold them: four in
+// blocks of 256 up to k r = 36, two in blocks of 128 up to k r = 73. The default block is the one with
+// four (5e6 photons of the precision scale-up: march kernel 273 ms with one copy, 264 with two in
+// blocks of 128, 254 with four in blocks of 256).
+static bool copies_fit(const smp_plan *p, int block) {
+    return p->fk <= FK_BESSELN && (p->smem_bytes * march_copies(block) + 1024) * size_t(6 * 128 / block) <= 220 * 1024;
+}
+static int march_block_default(const smp_plan *p) { return copies_fit(p, 256) ? 256 : 128; }
+
 static int wave_setup(smp_plan *p) {
     const bool bricks = p->fk == FK_SPLINE && p->bricks;
-    // copies of the Bessel table (dev_field.cuh RepTable) as long as the SM's resident blocks hold them:
-    // four in blocks of 256 up to k r = 36, two up to k r = 73, of which an untuned plan takes the first
-    // (5e6 photons of the precision scale-up: march kernel 273 ms with one copy, 264 with two in blocks
-    // of 128, 254 with four in blocks of 256)
-    auto fits = [p](int block) {
-        return p->fk <= FK_BESSELN && (p->smem_bytes * march_copies(block) + 1024) * size_t(6 * 128 / block) <= 220 * 1024;
-    };
-    if (!p->tuned && !p->block_fixed) p->march_block = fits(256) ? 256 : 128;
-    p->march_copies = fits(p->march_block) ? march_copies(p->march_block) : 1;
+    if (!p->tuned && !p->block_fixed) p->march_block = march_block_default(p);
+    p->march_copies = copies_fit(p, p->march_block) ? march_copies(p->march_block) : 1;
     WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, bricks, p->march_copies), fe = wf_event_fn(p->fk);
     if (!fm || !fe) return set_error(SMP_ERR_BAD_ARG, "bad field kind");
     p->march_smem = bricks ? size_t(kBrickSmemBytes) : p->smem_bytes * size_t(p->march_copies);
@@ -1436,7 +1438,8 @@ static int plan_tune(smp_plan *plan, int64_t n_sample, int64_t n_grow, smp_tunin
     double ms = 0.0;
     smp_tuning t;
     std::memset(&t, 0, sizeof(t));
-    t.march_block = 128; t.slots_per_lane = kSlots[0]; t.chunk = kChunks[1];
+    const int block0 = march_block_default(plan);
+    t.march_block = block0; t.slots_per_lane = kSlots[0]; t.chunk = kChunks[1];
     tune_apply(plan, t);
     // warm-up (allocations, module load) on at most 2e5 photons, which also measures the rate
     const int64_t n_warm = std::min<int64_t>(n_sample, 200000);
@@ -1472,7 +1475,7 @@ static int plan_tune(smp_plan *plan, int64_t n_sample, int64_t n_grow, smp_tunin
             consider(t, ms);
         }
     t = best;
-    t.march_block = 256;
+    t.march_block = block0 == 256 ? 128 : 256;
     tune_apply(plan, t);
     rc = tune_trial(plan, n_sample, weight, &ms);
     if (rc) return rc;

@@ -14,7 +14,6 @@
 // splats and end state with the CPU restatement on injected uniform streams.
 #pragma once
 #include <cooperative_groups.h>
-#include <cooperative_groups/reduce.h>
 
 #include <climits>
 #include <type_traits>
@@ -973,8 +972,8 @@ static __device__ __noinline__ bool stage_to_shared(void *dst, const void *src, 
 
 // The lane loop of the persistent kernel: event phase (lanes whose march ended, or that need a
 // photon, run their discrete logic together until every live lane marches again; photons come
-// from the global counter, one atomic per warp) alternating with the march phase (two ER steps per
-// vote until event_batch lanes, scaled by the live lanes, wait for events). A lane enters with
+// from the global counter, one atomic per warp) alternating with the march phase (an untested window or
+// eight ER steps per vote until event_batch lanes, scaled by the live lanes, wait for events). A lane enters with
 // `st` = ST_FETCH (no photon) or ST_MARCH (a photon loaded mid-march). All 32 lanes call it.
 // A hook (adjoint.cuh's checkpointing trace) also sees each photon's start and end; the render
 // kernels use NoHook.
