@@ -378,12 +378,13 @@ static void fill_field_params(const smp_field_desc &f, int fk, FieldParams &F) {
     F.binv_h = float(1.0 / kBesselH);
     F.kb = F.k_r * F.binv_h;
     // Bounds for the march's untested windows (the spline's come with its coefficients). Bessel, with
-    // |s| <= 1 (the clamp is at max_scaling; a negative one could let s past 1, then no bounds):
+    // |s| <= 1 (the clamp is at max_scaling; a negative one could let s past 1, and a phase that is not
+    // finite takes s to the clamp itself, which may lie beyond 1: then no bounds):
     // |n - n_o| <= |A|; |dn/dr| <= |A| k |J_m'| <= |A| k and |dn/(r dphi)| = |A| k m |J_m(x)|/x
     // <= |A| k, so |grad n|_1 <= 2 |A| k, twice that for the table's interpolation error. Plane waves:
     // sum |a_i| and sum |a_i| |k_i|_1.
     double dev = -1.0, grad = 0.0;
-    if (fk <= FK_BESSELN && !(F.max_scaling < 0.0f)) {
+    if (fk <= FK_BESSELN && !(F.max_scaling < 0.0f) && std::isfinite(F.phi_min) && std::isfinite(F.phi_range)) {
         dev = std::fabs(double(F.amp));
         grad = 4.0 * dev * double(F.k_r);
     }

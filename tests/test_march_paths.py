@@ -211,3 +211,41 @@ def test_prefilter_shapes_against_the_oracle(shape):
     ref, s64 = np.zeros(s.size), s.astype(np.float64)
     ob.oracle().orc_spline_prefilter3d(p(s64), p(n), 32, p(ref))
     assert np.allclose(got.reshape(-1), ref, rtol=0, atol=2e-6)
+
+
+NAN = float("nan")
+NON_FINITE = {
+    "wave_phase": lambda: sb.config_planewave(wave_phase=(NAN, 0.3), seed=50),
+    "wave_tau": lambda: sb.config_planewave(phi_min=NAN, seed=51, **MIXED),
+    "wave_tau_past_the_gap": lambda: sb.config_planewave(phi_min=NAN, emitter_gap=2e-3, seed=52),
+    "distance": lambda: sb.config_plain_small(mode=1, sigma_t=NAN, seed=53),
+    # a phase that is not a number takes the scaling to the clamp: a finite field fifty times the amplitude,
+    # lowest near the side faces (k r = 3.8)
+    "clamp_past_the_amplitude": lambda: sb.config_plain_small(mode=0, n_max=0.01, n_clip=0.5, f_u=180e3, phi_min=NAN,
+                                                              seed=54),
+}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(NON_FINITE))
+def test_non_finite_photons_end_as_the_plain_kernels(name, monkeypatch):
+    """No untested window for a state that is not finite: end codes, step counts and the call's status of the
+    one launch, the pool with its tail and the persistent kernel are the plain kernel's."""
+    import ctypes as C
+    s = dataclasses.replace(NON_FINITE[name](), sensor_march_max=0.05, max_depth=4)
+
+    def trace(s, n=300):
+        recs = (L.PhotonRecord * n)()
+        sc, md, fd, op = s.descs()
+        rc = sb.load().smp_trace_photons(C.byref(sc), C.byref(md), C.byref(fd), C.byref(op), 0, n, n, None, None, recs, None)
+        return rc, sb.records_to_arrays(recs)
+
+    rc0, ref = trace(dataclasses.replace(s, kernel=L.KERNEL_PLAIN))
+    assert rc0 == (L.SMP_ERR_NAN if name.startswith("wave") else L.SMP_OK)
+    for kernel, direct in ((L.KERNEL_POOL, "1000000"), (L.KERNEL_POOL, "0"), (L.KERNEL_PERSISTENT, "0")):
+        monkeypatch.setenv("SMP_WF_DIRECT", direct)
+        rc, got = trace(dataclasses.replace(s, kernel=kernel))
+        assert rc == rc0
+        for f in ("end", "er_steps", "draws", "depth", "n_splats"):
+            assert np.array_equal(got[f], ref[f]), (name, kernel, direct, f)
+        assert np.array_equal(got["pos"], ref["pos"], equal_nan=True)
