@@ -19,6 +19,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -428,15 +429,22 @@ static void set_step_sizes(KParams &k, const smp_field_desc &f) {
     step_table(f.er_stepsize, k.cur_tab);
 }
 
-// Runs f(begin, end) over [0, n) on up to 16 host threads.
+// Runs f(begin, end) over [0, n) on up to 16 host threads; where a thread cannot be had (a limit on
+// threads or address space), this one does the rest.
 template <class F>
 static void host_parallel(size_t n, F f) {
     const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
     const size_t per = (n + hw - 1) / hw;
     std::vector<std::thread> ts;
-    for (unsigned t = 0; t < hw; ++t) {
-        const size_t a = std::min(n, t * per), b = std::min(n, a + per);
-        if (a < b) ts.emplace_back([&f, a, b] { f(a, b); });
+    ts.reserve(hw);
+    size_t a = 0;
+    try {
+        for (; a < n; a += per) {
+            const size_t b = std::min(n, a + per);
+            ts.emplace_back([&f, a, b] { f(a, b); });
+        }
+    } catch (const std::system_error &) {
+        f(a, n);
     }
     for (auto &t : ts) t.join();
 }

@@ -249,3 +249,27 @@ def test_non_finite_photons_end_as_the_plain_kernels(name, monkeypatch):
         for f in ("end", "er_steps", "draws", "depth", "n_splats"):
             assert np.array_equal(got[f], ref[f]), (name, kernel, direct, f)
         assert np.array_equal(got["pos"], ref["pos"], equal_nan=True)
+
+
+def test_prefilter_without_room_for_threads():
+    """A process that cannot start another thread (here: no address space for its stack) still gets its
+    coefficients, the same ones."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import ctypes as C, resource, numpy as np, simpler_b200 as sb
+lib, p = sb.load(), lambda a: C.c_void_p(a.ctypes.data)
+s = np.random.default_rng(1).standard_normal((96, 40, 64)).astype(np.float32)
+n, free, tight = np.array((64, 40, 96), np.int32), np.zeros_like(s), np.zeros_like(s)
+vm = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+soft, hard = resource.getrlimit(resource.RLIMIT_AS)
+resource.setrlimit(resource.RLIMIT_AS, (vm + (1 << 20), hard))      # before any thread leaves its stack behind
+assert lib.smp_spline_prefilter(p(s), p(n), p(tight)) == 0
+resource.setrlimit(resource.RLIMIT_AS, (soft, hard))
+assert lib.smp_spline_prefilter(p(s), p(n), p(free)) == 0
+assert np.array_equal(free, tight)
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-500:]
