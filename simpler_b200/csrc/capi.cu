@@ -115,17 +115,20 @@ static void prefilter_1d(const float *data, long off, long stride, int size, con
     }
 }
 
-template <class F> static void host_parallel(size_t n, F f);
+template <class F> static void host_parallel(size_t n, size_t grain, F f);
 
 // Spline<3>::build3d (spline.h:739-764): y, then x, then z passes; the lines of a pass are independent
 // and run on the host's threads
+// where a share is worth its thread: a thread costs 30 to 100 us, and 16,384 samples of a pass about 100.
+// 8^3 samples: 25 us on the caller's thread, 560 on sixteen; 64^3: 5 ms on one, 1.9 on sixteen.
+static const size_t kPrefilterGrain = 16384;
 static void prefilter_3d(const float *samples, const int N[3], float *coeff) {
     const long s01 = long(N[0]) * N[1];
     auto pass = [&](const float *src, int axis, int other, long sa, long s1, int outer, long s2) {
         // lines along `axis` of stride sa: `outer` planes of stride s2, N[other] lines of stride s1
         const int size = N[axis];
         const std::vector<float> pw = prefilter_powers(size);
-        host_parallel(size_t(outer) * N[other], [&, size](size_t a, size_t b) {
+        host_parallel(size_t(outer) * N[other], std::max<size_t>(1, kPrefilterGrain / size), [&, size](size_t a, size_t b) {
             std::vector<float> tmp(2 * size_t(size));
             for (size_t l = a; l < b; ++l) {
                 const long off = long(l / N[other]) * s2 + long(l % N[other]) * s1;
@@ -429,15 +432,16 @@ static void set_step_sizes(KParams &k, const smp_field_desc &f) {
     step_table(f.er_stepsize, k.cur_tab);
 }
 
-// Runs f(begin, end) over [0, n) on up to 16 host threads; where a thread cannot be had (a limit on
-// threads or address space), this one does the rest.
+// Runs f(begin, end) over [0, n) on up to 16 host threads, each with at least `grain` of it (the caller's
+// own share first of all: one share is no thread); where a thread cannot be had (a limit on threads or
+// address space), the caller does the rest.
 template <class F>
-static void host_parallel(size_t n, F f) {
-    const unsigned hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    const size_t per = (n + hw - 1) / hw;
+static void host_parallel(size_t n, size_t grain, F f) {
+    const size_t hw = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+    const size_t shares = std::max<size_t>(1, std::min(hw, n / grain)), per = (n + shares - 1) / shares;
     std::vector<std::thread> ts;
-    ts.reserve(hw);
-    size_t a = 0;
+    ts.reserve(shares);
+    size_t a = per;
     try {
         for (; a < n; a += per) {
             const size_t b = std::min(n, a + per);
@@ -446,6 +450,7 @@ static void host_parallel(size_t n, F f) {
     } catch (const std::system_error &) {
         f(a, n);
     }
+    f(0, std::min(n, per));
     for (auto &t : ts) t.join();
 }
 
@@ -1901,17 +1906,17 @@ int smp_render_batch(const smp_scene_desc *scene, const smp_instance_desc *insta
         cudaError_t e;
         if (opts->precision == SMP_PREC_MIXED) {
             const size_t cnt = fb / 8 * size_t(n_inst);
-            host_parallel(cnt, [images_out](size_t a, size_t b) { std::memset(images_out + a, 0, (b - a) * 8); });
+            host_parallel(cnt, 1, [images_out](size_t a, size_t b) { std::memset(images_out + a, 0, (b - a) * 8); });
             e = cudaMemcpy(images_out, d_films, cnt * 8, cudaMemcpyDeviceToHost);
         } else {
             // FP32 films through a staging buffer, widened on the host by several threads
             const size_t cnt = fb / 4 * size_t(n_inst);
             std::unique_ptr<float[]> h(new float[cnt]);
             float *hp = h.get();
-            host_parallel(cnt, [hp](size_t a, size_t b) { std::memset(hp + a, 0, (b - a) * 4); });
+            host_parallel(cnt, 1, [hp](size_t a, size_t b) { std::memset(hp + a, 0, (b - a) * 4); });
             e = cudaMemcpy(hp, d_films, cnt * 4, cudaMemcpyDeviceToHost);
             if (e == cudaSuccess)
-                host_parallel(cnt, [hp, images_out](size_t a, size_t b) {
+                host_parallel(cnt, 1, [hp, images_out](size_t a, size_t b) {
                     for (size_t j = a; j < b; ++j) images_out[j] = double(hp[j]);
                 });
         }

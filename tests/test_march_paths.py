@@ -273,3 +273,22 @@ assert np.array_equal(free, tight)
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-500:]
+
+
+def test_small_prefilters_start_no_threads():
+    """4^3 samples against 24^3, 216 times the work and on one thread as well: half its time at most. (Threads
+    for either cost several hundred microseconds, many times the small one's work.)"""
+    import ctypes as C
+    import time
+    lib, p = sb.load(), lambda a: C.c_void_p(a.ctypes.data)
+
+    def best(size):
+        s = np.random.default_rng(3).standard_normal((size,) * 3).astype(np.float32)
+        n, out, t = np.full(3, size, np.int32), np.zeros_like(s), []
+        for _ in range(50):
+            t0 = time.perf_counter()
+            L.check(lib.smp_spline_prefilter(p(s), p(n), p(out)))
+            t.append(time.perf_counter() - t0)
+        return min(t)
+
+    assert best(4) <= 0.5 * best(24)
