@@ -292,3 +292,22 @@ def test_small_prefilters_start_no_threads():
         return min(t)
 
     assert best(4) <= 0.5 * best(24)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel", [L.KERNEL_PERSISTENT, L.KERNEL_POOL])
+def test_lone_point_source_steps(kernel):
+    """A lone photon's step of the point-source field is its sum over the sources, whose latency the lane loop
+    hides as well as two steps in a straight line let it: 0.36 (persistent) and 0.41 (one launch) of the plain
+    kernel's time for the same photons, 0.55 with a step a turn. The limit is half way."""
+    s = sb.config_sources(theta_sources=20, trans_z_sources=50, er_stepsize=4e-4, sensor_march_max=0.1, seed=3,
+                          spatial_x=64, spatial_y=64, path_length_bins=8)
+
+    def best(kernel):
+        plan = sb.Plan(dataclasses.replace(s, kernel=kernel))
+        try:
+            return min(plan.render(8)[1].kernel_ms for _ in range(4))
+        finally:
+            plan.close()
+
+    assert best(kernel) <= 0.48 * best(L.KERNEL_PLAIN)
