@@ -2288,9 +2288,11 @@ static cudaError_t adjoint_trace_pool(smp_plan *p, const KParams &k, const AdjPa
     W.nb = 0;
     WaveFn fm = wf_march_fn(p->fk, p->kp.fp64 != 0, p->march_block, false, p->march_copies);
     if (!fm) return cudaErrorInvalidDeviceFunction;
-    if (p->march_smem > 48 * 1024) {
+    // of the kernel launched here: a plan with bricks has their size in march_smem
+    const size_t smem = p->smem_bytes * size_t(p->march_copies);
+    if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void *>(fm), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             int(p->march_smem));
+                                             int(smem));
         if (e != cudaSuccess) return e;
     }
     const unsigned finish_at = unsigned(grid_f) * unsigned(kBlock);
@@ -2304,7 +2306,7 @@ static cudaError_t adjoint_trace_pool(smp_plan *p, const KParams &k, const AdjPa
     int par = 0;
     for (;;) {
         for (int j = 0; j < p->wave_batch; ++j, ++it) {
-            fm<<<p->grid_march, p->march_block, p->march_smem>>>(k, W, int(it & 0x3fffffff));
+            fm<<<p->grid_march, p->march_block, smem>>>(k, W, int(it & 0x3fffffff));
             fe<<<p->grid_event, kBlock>>>(k, W, a, int(it & 0x3fffffff));
         }
         *launches += 2 * p->wave_batch;

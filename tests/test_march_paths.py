@@ -311,3 +311,24 @@ def test_lone_point_source_steps(kernel):
             plan.close()
 
     assert best(kernel) <= 0.48 * best(L.KERNEL_PLAIN)
+
+
+@pytest.mark.gpu
+def test_adjoint_of_a_brick_plan_marches_without_the_bricks_memory(tmp_path):
+    """The adjoint's trace of a plan with coefficient bricks launches the march kernel without bricks, which uses
+    no shared memory of its own: the bricks' 92 KB a block would only take its L1 cache."""
+    import json
+
+    import torch
+    s = sb.config_spline(16, 4, spline_bricks=True, spatial_x=64, spatial_y=64, path_length_bins=4)
+    plan = sb.Plan(s)
+    try:
+        plan.adjoint(sb.roi_weights(s, 32), 0, 100)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            plan.adjoint(sb.roi_weights(s, 32), 0, 100)
+    finally:
+        plan.close()
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+    marches = [e["args"] for e in events if e.get("cat") == "kernel" and "wf_march_kernel" in e["name"]]
+    assert marches and all(m["shared memory"] < 16384 for m in marches), marches[:1]
