@@ -250,7 +250,7 @@ template <int NW> struct FieldAdjPW {
             if (i < F.n_waves) {
                 const float kx = F.wk[i][0], ky = F.wk[i][1], kz = F.wk[i][2];
                 float sn, cs;
-                sincos_red(kx * p.x + ky * p.y + kz * p.z - tau + F.wphase[i], sn, cs);
+                sincos_near(kx * p.x + ky * p.y + kz * p.z - tau + F.wphase[i], sn, cs);
                 n += F.wamp[i] * sn;
                 const float ac = F.wamp[i] * cs, as = -F.wamp[i] * sn;
                 g.x += ac * kx; g.y += ac * ky; g.z += ac * kz;
@@ -266,7 +266,7 @@ template <int NW> struct FieldAdjPW {
             if (i < F.n_waves) {
                 const float kx = F.wk[i][0], ky = F.wk[i][1], kz = F.wk[i][2];
                 float sn, cs;
-                sincos_red(kx * p.x + ky * p.y + kz * p.z - tau + F.wphase[i], sn, cs);
+                sincos_near(kx * p.x + ky * p.y + kz * p.z - tau + F.wphase[i], sn, cs);
                 const float kb = kx * b.x + ky * b.y + kz * b.z;
                 c.ga[i] += a * sn + cs * kb;
                 c.gp[i] += F.wamp[i] * (a * cs - sn * kb);
@@ -287,7 +287,7 @@ template <int NW> struct FieldAdjPW {
             if (i < F.n_waves) {
                 const float kx = F.wk[i][0], ky = F.wk[i][1], kz = F.wk[i][2];
                 float sn, cs;
-                sincos_red(kx * p.x + ky * p.y + kz * p.z - tau + F.wphase[i], sn, cs);
+                sincos_near(kx * p.x + ky * p.y + kz * p.z - tau + F.wphase[i], sn, cs);
                 k.sn[i] = sn; k.cs[i] = cs;
                 n += F.wamp[i] * sn;
                 const float ac = F.wamp[i] * cs, as = -F.wamp[i] * sn;
@@ -1299,7 +1299,7 @@ __device__ __forceinline__ void job_after(PhotonJobs &J, Lane &L, const KParams 
             }
             const float sinT = sqrtf(fmaxf(0.0f, 1.0f - cosT * cosT));
             float sP, cP;
-            sincos_red(6.28318548202514648f * u2, sP, cP);
+            sincos_near(6.28318548202514648f * u2, sP, cP);
             J.ld = hg_vjp(f3(c.dir[0], c.dir[1], c.dir[2]), cosT, sinT, cP, sP, w.Da);
         } else {
             J.ld = w.Da;

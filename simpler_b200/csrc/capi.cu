@@ -344,6 +344,12 @@ static int field_kind(const smp_field_desc &f, int *fk) {
     }
 }
 
+// A phase without its whole turns, if it has more than ten of them: added to k p in float it would take that
+// sum's low bits (all of them from 1e7 turns on), and its sine's argument could pass sincos_near's range.
+static float near_phase(float x) {
+    return std::fabs(x) > 64.0f && std::isfinite(x) ? float(std::remainder(double(x), 6.283185307179586)) : x;
+}
+
 // float field parameters shared by plans and probes (device pointers filled by the caller)
 static void fill_field_params(const smp_field_desc &f, int fk, FieldParams &F) {
     std::memset(&F, 0, sizeof(F));
@@ -360,10 +366,11 @@ static void fill_field_params(const smp_field_desc &f, int fk, FieldParams &F) {
     F.max_scaling = float(f.n_clip) / float(f.n_max);       // rif_analytical.h:222
     F.phi_min = float(f.phi_min);
     F.phi_range = float(f.phi_max) - float(f.phi_min);
+    if (fk == FK_PLANEWAVE) F.phi_min = near_phase(F.phi_min);
     F.n_waves = f.n_waves;
     for (int i = 0; i < SMP_MAX_WAVES && i < f.n_waves; ++i) {
         F.wamp[i] = float(f.wave_amp[i]);
-        F.wphase[i] = float(f.wave_phase[i]);
+        F.wphase[i] = near_phase(float(f.wave_phase[i]));
         for (int j = 0; j < 3; ++j) F.wk[i][j] = float(f.wave_k[i][j]);
     }
     F.n_coeff = f.n_coeff;
@@ -371,8 +378,8 @@ static void fill_field_params(const smp_field_desc &f, int fk, FieldParams &F) {
     F.active1 = f.active1;
     F.active2 = f.active2;
     F.n_scaling = float(f.n_scaling);
-    F.phase1 = float(f.phase1);
-    F.phase2 = float(f.phase2);
+    F.phase1 = near_phase(float(f.phase1));
+    F.phase2 = near_phase(float(f.phase2));
     for (int i = 0; i < 3; ++i) {
         F.N[i] = f.grid_n[i];
         F.xmin[i] = float(f.grid_min[i]);

@@ -188,7 +188,7 @@ __device__ __forceinline__ void wave_field_ng(const FieldParams &F, float3 p, fl
         if (i >= F.n_waves) break;
         float ph = F.wk[i][0] * p.x + F.wk[i][1] * p.y + F.wk[i][2] * p.z - tau + F.wphase[i];
         float sn, cs;
-        sincos_red(ph, sn, cs);
+        sincos_near(ph, sn, cs);
         acc = fmaf(F.wamp[i], sn, acc);
         float ac = F.wamp[i] * cs;
         gg.x = fmaf(ac, F.wk[i][0], gg.x);
@@ -237,7 +237,7 @@ __device__ __forceinline__ void sources_field(const FieldParams &F, float3 p, fl
                 float r = rr2 * ir;
                 float krc = F.k_r * r * float(c);
                 float sn, cs;
-                sincos_red(krc + ph, sn, cs);
+                sincos_near(krc + ph, sn, cs);
                 trif = fmaf(cs, ir, trif);
                 float ct = -fmaf(krc, sn, cs) * ir * ir * ir;
                 tdn.x = fmaf(ct, dx, tdn.x);

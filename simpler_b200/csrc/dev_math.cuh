@@ -67,18 +67,25 @@ __device__ __forceinline__ int floor_frac(float t, float &frac) {
 __device__ __forceinline__ float comp(float3 a, int i) { return i == 0 ? a.x : (i == 1 ? a.y : a.z); }
 __device__ __forceinline__ float3 ld3(const float *v) { return f3(v[0], v[1], v[2]); }
 
-// sin and cos of an argument of moderate size (|t| < 1e4): Cody-Waite reduction by 2*pi with a
-// two-term split of 2*pi, then the hardware approximations on [-pi, pi].
-__device__ __forceinline__ void sincos_red(float t, float &s, float &c) {
-    const float kInv2Pi = 0.159154943091895335768f;
+// sin and cos by Cody-Waite reduction by 2*pi with a two-term split of 2*pi, then the hardware
+// approximations on [-pi, pi]. q: t / (2 pi) rounded to an integer.
+static constexpr float kInv2Pi = 0.159154943091895335768f;
+__device__ __forceinline__ void sincos_cw(float t, float q, float &s, float &c) {
     const float k2PiHi = 6.28318548202514648438f;     // float(2*pi)
     const float k2PiLo = -1.74845553146951609e-07f;   // 2*pi - float(2*pi)
-    // rintf by an add that rounds to an integer (two adds instead of a conversion-pipe instruction, which
-    // shares its pipe with the sine and cosine)
-    float q = (t * kInv2Pi + 12582912.0f) - 12582912.0f;
     float r = fmaf(-q, k2PiHi, t);
     r = fmaf(-q, k2PiLo, r);
     __sincosf(r, &s, &c);
+}
+// an argument of any size (to 1e-6 at 2e8)
+__device__ __forceinline__ void sincos_red(float t, float &s, float &c) { sincos_cw(t, rintf(t * kInv2Pi), s, c); }
+// |t| <= 2.6e7 (2^22 turns): rintf, to the bit, by an add that rounds to an integer, two adds instead of a
+// conversion-pipe instruction, which shares its pipe with the sine and cosine (a lone plane-wave step 136
+// to 128 ns). Past that q may be off by half a turn; a float sum that large has lost its turn anyway (its
+// last place is 2), and the host takes the turns out of large phases (capi.cu near_phase). A test of every
+// argument here cost a lone step 16 %, the plane-wave march 4 to 10 %, the source sums 12 to 30 %.
+__device__ __forceinline__ void sincos_near(float t, float &s, float &c) {
+    sincos_cw(t, (t * kInv2Pi + 12582912.0f) - 12582912.0f, s, c);
 }
 
 template <int M> struct BesselSeries;

@@ -315,7 +315,7 @@ __device__ __forceinline__ float3 hg_sample(Lane &L, const KParams &P, float3 in
     float sinT = sqrtf(fmaxf(0.0f, 1.0f - cosT * cosT));
     float phi = 6.28318548202514648f * sy;
     float sP, cP;
-    sincos_red(phi, sP, cP);
+    sincos_near(phi, sP, cP);
     float3 ax, ay;
     if (fabsf(in.x) > fabsf(in.y)) {
         float inv = 1.0f / sqrtf(in.x * in.x + in.z * in.z);
@@ -335,7 +335,7 @@ __device__ __forceinline__ float3 random_direction(Lane &L, const KParams &P) {
     float ux = draw(L, P);
     float tmp = sqrtf(1.0f - ux * ux);
     float sP, cP;
-    sincos_red(6.28318548202514648f * uy, sP, cP);
+    sincos_near(6.28318548202514648f * uy, sP, cP);
     return f3(-ux, cP * tmp, sP * tmp);
 }
 
@@ -374,7 +374,7 @@ __device__ __forceinline__ bool gen_ray(Lane &L, const KParams &P, float3 &pos, 
     float zt = sqrtf(1.0f - z * z);
     float phi = draw(L, P) * 2.0f * 3.14159265358979f;
     float sP, cP;
-    sincos_red(phi, sP, cP);
+    sincos_near(phi, sP, cP);
     dir = f3(-z, zt * cP, zt * sP);
     // Lens::propagate_till_lens (lens.cpp:20-33)
     float dist = -(pos.x - P.src_lens_origin[0]) / dir.x;
@@ -1148,7 +1148,7 @@ sources_values_kernel(const __grid_constant__ FieldParams F, int nt, long long n
                 const float r = rr2 * ir;
                 const float krc = F.k_r * r * fc;
                 float sn, cs;
-                sincos_red(krc + ph, sn, cs);
+                sincos_near(krc + ph, sn, cs);
                 trif = fmaf(cs, ir, trif);
             };
             for (int j = 0; j < nz; ++j) {

@@ -332,3 +332,53 @@ def test_adjoint_of_a_brick_plan_marches_without_the_bricks_memory(tmp_path):
     events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
     marches = [e["args"] for e in events if e.get("cat") == "kernel" and "wf_march_kernel" in e["name"]]
     assert marches and all(m["shared memory"] < 16384 for m in marches), marches[:1]
+
+
+def turns(n, fraction):
+    """The float nearest to n + fraction turns, an argument that rounds to n or n + 1 of them."""
+    import math
+    x = np.float32((n + fraction) * 2.0 * math.pi)
+    return float(min((np.nextafter(x, np.float32(s * np.inf)) if s else x for s in (-1, 0, 1)),
+                     key=lambda y: abs(abs(math.remainder(float(y), 2.0 * math.pi)) - abs(fraction) * 2.0 * math.pi)))
+
+
+FAR = {
+    "bessel": lambda ph: sb.config_plain_small(mode=0, n_max=0.05, n_clip=0.05, phi_min=ph, phi_max=ph),
+    "wave": lambda ph: sb.config_planewave(wave_amp=(0.03, 0.02), wave_k=((0.0, 3e2, 0.0), (0.0, 0.0, 4e2)),
+                                           wave_phase=(ph, -ph)),
+    "wave_tau": lambda ph: sb.config_planewave(wave_amp=(0.05,), wave_k=((0.0, 3e2, 0.0),), wave_phase=(0.25,),
+                                               phi_min=ph, phi_max=ph),
+    "sources": lambda ph: sb.config_sources(theta_sources=6, trans_z_sources=3, n_scaling=2e-3, phase1=ph, phase2=-ph,
+                                            er_stepsize=1e-4),
+}
+PHASES = {"bessel": ("phi_min", "phi_max"), "wave": ("wave_phase",), "wave_tau": ("phi_min", "phi_max"),
+          "sources": ("phase1", "phase2")}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kernel", [L.KERNEL_POOL, L.KERNEL_PLAIN])
+@pytest.mark.parametrize("n", [-7900001, -5000003, 5000003, 11000000, -1000])
+@pytest.mark.parametrize("name", sorted(FAR))
+def test_phases_of_many_turns(name, n, kernel):
+    """A phase of millions of turns (a time of seconds, in radians) gives the field of its remainder. A sine is good to
+    1e-6 there, so the index is to 1e-6 of the amplitude, 0.05, and the direct light's optical path, whose steps add in
+    double, to 1e-5 of itself; half a turn too much moves it by 1e-3 or more."""
+    import ctypes as C
+    import math
+    far = FAR[name](turns(n, 0.42))
+    one = lambda x: math.remainder(x, 2.0 * math.pi)      # noqa: E731
+    near = dataclasses.replace(far, **{f: tuple(map(one, v)) if isinstance(v := getattr(far, f), tuple) else one(v)
+                                       for f in PHASES[name]})
+    paths = []
+    for s in (far, near):
+        s = dataclasses.replace(s, albedo=0.0, kernel=kernel, **MIXED)
+        recs, _ = sb.trace_photons(s, 0, 200, 200, with_image=False)
+        paths.append(sb.records_to_arrays(recs)["total_optical"])
+    assert np.allclose(paths[0], paths[1], rtol=1e-5, atol=0)
+    if name == "sources" and kernel == L.KERNEL_POOL:
+        pts = np.ascontiguousarray(np.random.default_rng(0).uniform(-5e-3, 5e-3, (300, 3)))
+        n_far, n_near = (sb.field_eval(s, 0.0, pts)[0] for s in (far, near))
+        assert np.abs(n_far - n_near).max() <= 1e-5 * np.abs(n_near - far.n_o).max() + 2e-7
+        got, fd = np.zeros(300), far.field_desc()
+        L.check(sb.load().smp_field_values(C.byref(fd), 0.0, 300, C.c_void_p(pts.ctypes.data), C.c_void_p(got.ctypes.data)))
+        assert np.array_equal(got, n_far)
