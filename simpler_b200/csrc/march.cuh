@@ -496,14 +496,12 @@ __device__ __forceinline__ int safe_steps(const S &L, const KParams &P, int cap)
     const float kx = __fdividef(mx, fmaf(q, fabsf(L.md.x) + kick, P.win_round));
     const float ky = __fdividef(my, fmaf(q, fabsf(L.md.y) + kick, P.win_round));
     const float kz = __fdividef(mz, fmaf(q, fabsf(L.md.z) + kick, P.win_round));
-    const float left = L.dlimit - L.dist_acc;
-    // Each bound on its own: a minimum would drop one that is not a number. A step with a momentum,
-    // position or n that is not finite moves nowhere, and march_step's tests end its march. (kd alone may
-    // be inf / inf, for a distance limit of inf.)
-    if (!((kx >= 1.0f) & (ky >= 1.0f) & (kz >= 1.0f) & (left > 0.0f) & (L.mn >= F.n_low))) return 0;
-    const float kd = __fdividef(left, fmaf(1.03f, h, 1.2e-7f * L.dlimit));
+    const float left = L.dlimit - L.dist_acc, kd = __fdividef(left, fmaf(1.03f, h, 1.2e-7f * L.dlimit));
     const float k = 0.999f * fminf(fminf(kx, ky), fminf(kz, kd));
-    if (!(k >= 1.0f)) return 0;                            // no room
+    // Room for a step, and a state that is finite: a minimum drops an operand that is not a number, a sum
+    // keeps it (kd alone may be inf / inf, for a distance limit of inf). A step from any other state moves
+    // nowhere, and march_step's tests end its march.
+    if (!((k >= 1.0f) & ((kx + ky) + kz >= 1.0f) & (left > 0.0f) & (L.mn >= F.n_low))) return 0;
     return min(int(fminf(k, float(cap))), L.stop - L.steps - 1);
 }
 
