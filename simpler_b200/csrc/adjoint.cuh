@@ -297,10 +297,6 @@ template <int NW> struct FieldAdjPW {
             }
         }
     }
-    static __device__ __forceinline__ void eval_s(const FieldParams &F, float3 p, float tau, float &n, float3 &g, float H[6],
-                                                  Cache &k, Acc &) {
-        eval_h(F, p, tau, n, g, H, k);
-    }
     static __device__ __forceinline__ void theta_c(const FieldParams &F, float3, float, float a, float3 b, Acc &c,
                                                    const AdjParams &, const Cache &k) {
         if (k.gap) return;
@@ -339,10 +335,7 @@ __device__ __forceinline__ void bspline_dd(float t, float dd[4]) {
     dd[3] = f;
 }
 template <> struct FieldAdj<FK_SPLINE> {
-    struct Acc { SplineCell C; };              // the tap rows of the sweep's current cell
-    struct Cache {};
-    static __device__ __forceinline__ void begin(Acc &, Lane &, const KParams &, float) {}
-    static __device__ __forceinline__ void clear(Acc &c) { c.C.clear(); }
+    struct Acc {};                             // the shares go to memory as they come
     static __device__ __forceinline__ void taps(const FieldParams &F, float3 p, float wx[4], float wy[4], float wz[4],
                                                 float dx[4], float dy[4], float dz[4], float ddx[4], float ddy[4],
                                                 float ddz[4], int ix[4], int iy[4], int iz[4]) {
@@ -366,36 +359,31 @@ template <> struct FieldAdj<FK_SPLINE> {
         bspline_dd(t1, ddy);
         bspline_dd(t2, ddz);
     }
-    // The sixteen rows come in one batch of independent loads, and in the sweep, where a cell's points
-    // follow one another, once per cell (SplineCell): loaded row by row behind a test each, they were a
-    // sweep's whole time (26 of 27 cycles per instruction waiting for them).
-    static __device__ __forceinline__ void eval_s(const FieldParams &F, float3 p, float, float &n, float3 &g, float H[6],
-                                                  Cache &, Acc &acc) {
+    // The sixteen rows come in one batch of independent loads: loaded row by row behind a test each, they
+    // were a sweep's whole time (26 of 27 cycles per instruction waiting for them).
+    static __device__ __forceinline__ void eval_h(const FieldParams &F, float3 p, float, float &n, float3 &g, float H[6]) {
 #pragma unroll
         for (int j = 0; j < 6; ++j) H[j] = 0.0f;
         if (in_gap(F, p)) { n = F.n_o; g = f3(0.0f, 0.0f, 0.0f); return; }
         const float t0 = (p.x - F.xmin[0]) * F.xres[0], t1 = (p.y - F.xmin[1]) * F.xres[1], t2 = (p.z - F.xmin[2]) * F.xres[2];
         float wx[4], wy[4], wz[4], dx[4], dy[4], dz[4], ddx[4], ddy[4], ddz[4];
         weights(t0, t1, t2, wx, wy, wz, dx, dy, dz, ddx, ddy, ddz);
-        SplineCell &C = acc.C;
         const int x = int(floorf(t0)), y = int(floorf(t1)), z = int(floorf(t2));
-        if ((x != C.x) | (y != C.y) | (z != C.z)) {
-            if (spline_on_quads(F, x, y, z)) {
-                spline_rows(F, x, y, z, C.q);
-            } else {
-                int ix[4];
+        float4 q[16];
+        if (spline_on_quads(F, x, y, z)) {
+            spline_rows(F, x, y, z, q);
+        } else {
+            int ix[4];
 #pragma unroll
-                for (int a = 0; a < 4; ++a) ix[a] = spline_wrap(x - 1 + a, F.N[0]);
+            for (int a = 0; a < 4; ++a) ix[a] = spline_wrap(x - 1 + a, F.N[0]);
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
+            for (int c = 0; c < 4; ++c)
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) {
-                        const float *row = F.coeff + spline_wrap(z - 1 + c, F.N[2]) * F.N[0] * F.N[1] +
-                                           spline_wrap(y - 1 + b, F.N[1]) * F.N[0];
-                        C.q[4 * c + b] = make_float4(__ldg(row + ix[0]), __ldg(row + ix[1]), __ldg(row + ix[2]), __ldg(row + ix[3]));
-                    }
-            }
-            C.x = x; C.y = y; C.z = z;
+                for (int b = 0; b < 4; ++b) {
+                    const float *row = F.coeff + spline_wrap(z - 1 + c, F.N[2]) * F.N[0] * F.N[1] +
+                                       spline_wrap(y - 1 + b, F.N[1]) * F.N[0];
+                    q[4 * c + b] = make_float4(__ldg(row + ix[0]), __ldg(row + ix[1]), __ldg(row + ix[2]), __ldg(row + ix[3]));
+                }
         }
         float v = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
         float hxx = 0.0f, hyy = 0.0f, hzz = 0.0f, hxy = 0.0f, hxz = 0.0f, hyz = 0.0f;
@@ -403,7 +391,7 @@ template <> struct FieldAdj<FK_SPLINE> {
         for (int c = 0; c < 4; ++c) {
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                const float r0 = C.q[4 * c + b].x, r1 = C.q[4 * c + b].y, r2 = C.q[4 * c + b].z, r3 = C.q[4 * c + b].w;
+                const float r0 = q[4 * c + b].x, r1 = q[4 * c + b].y, r2 = q[4 * c + b].z, r3 = q[4 * c + b].w;
                 const float sv = r0 * wx[0] + r1 * wx[1] + r2 * wx[2] + r3 * wx[3];
                 const float sd = r0 * dx[0] + r1 * dx[1] + r2 * dx[2] + r3 * dx[3];
                 const float sdd = r0 * ddx[0] + r1 * ddx[1] + r2 * ddx[2] + r3 * ddx[3];
@@ -419,12 +407,6 @@ template <> struct FieldAdj<FK_SPLINE> {
         g = f3(gx * r0, gy * r1, gz * r2);
         H[0] = hxx * r0 * r0; H[1] = hyy * r1 * r1; H[2] = hzz * r2 * r2;
         H[3] = hxy * r0 * r1; H[4] = hxz * r0 * r2; H[5] = hyz * r1 * r2;
-    }
-    static __device__ __forceinline__ void eval_h(const FieldParams &F, float3 p, float s, float &n, float3 &g, float H[6]) {
-        Acc a;
-        a.C.clear();
-        Cache k;
-        eval_s(F, p, s, n, g, H, k, a);
     }
     static __device__ __forceinline__ void theta(const FieldParams &F, float3 p, float, float a, float3 b, Acc &, const AdjParams &A) {
         if (in_gap(F, p)) return;
@@ -444,11 +426,6 @@ template <> struct FieldAdj<FK_SPLINE> {
             }
         }
     }
-    static __device__ __forceinline__ void theta_c(const FieldParams &F, float3 p, float s, float a, float3 b, Acc &c,
-                                                   const AdjParams &A, const Cache &) {
-        theta(F, p, s, a, b, c, A);
-    }
-    static __device__ __forceinline__ void flush(const Acc &, const FieldParams &, const AdjParams &) {}
 };
 
 // ---- replay hook: checkpoints (phase A), stop at a segment's end (phase B), splat capture ----------
@@ -512,10 +489,6 @@ template <int M> struct FieldAdjBessel {
     }
     static __device__ __forceinline__ void eval_h(const FieldParams &F, float3 p, float s, float &n, float3 &g, float H[6]) {
         Cache k;
-        eval_h(F, p, s, n, g, H, k);
-    }
-    static __device__ __forceinline__ void eval_s(const FieldParams &F, float3 p, float s, float &n, float3 &g, float H[6],
-                                                  Cache &k, Acc &) {
         eval_h(F, p, s, n, g, H, k);
     }
     static __device__ __forceinline__ void theta_c(const FieldParams &, float3, float, float a, float3 b, Acc &c,
@@ -740,7 +713,7 @@ __device__ __forceinline__ void sweep_begin(Sweep &w, const KParams &P, const Ad
     float n_k, H[6];
     float3 g_k, b;
     typename FA::Cache kc;
-    FA::eval_s(F, pk, s, n_k, g_k, H, kc, acc);
+    FA::eval_h(F, pk, s, n_k, g_k, H, kc);
     sweep_begin_at(w, P, pk, w.e.w, n_k, g_k, H, md_end, Pa, Da, a_end, T, face_end, b);
     FA::theta_c(F, pk, s, a_end, b, acc, A, kc);
 }
@@ -803,7 +776,7 @@ __device__ __forceinline__ int sweep_point(Sweep &w, const KParams &P, const Adj
     float n1, a1, H[6];
     float3 g1, b1;
     typename FA::Cache kc;
-    FA::eval_s(F, pp, s, n1, g1, H, kc, acc);
+    FA::eval_h(F, pp, s, n1, g1, H, kc);
     sweep_update(w, P, w.e.w, pp, pe.w, junction, n1, g1, H, a1, b1);
     if (pe.w == 0.0f) return 1;
     FA::theta_c(F, pp, s, a1, b1, acc, A, kc);
@@ -1437,12 +1410,9 @@ __device__ __forceinline__ int warp_sweep(Sweep &w, const KParams &P, const AdjP
         const float3 pe = f3(e.x, e.y, e.z);
         float n = 1.0f, H[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, ta = 0.0f;
         float3 g = f3(0.0f, 0.0f, 0.0f), tb = g;
-        FA::Cache kc;
         bool use = false;
         if (idx >= 0 && (e.w >= 0.0f || idx == len - 1)) {
-            FA::Acc cell;
-            FA::clear(cell);
-            FA::eval_s(F, pe, s, n, g, H, kc, cell);
+            FA::eval_h(F, pe, s, n, g, H);
         }
         const int cnt = min(32, hi + 1);
         int res = 0;
@@ -1513,7 +1483,6 @@ static __global__ void __launch_bounds__(128, 3) adjoint_sweep_warp_kernel(const
         if (r.round != round) continue;
         L.idx = P.first_photon + k;
         FA::Acc acc;
-        FA::clear(acc);
         PhotonJobs J;
         job_photon(J, A, r);
         while (J.job != JOB_SOURCE) {
