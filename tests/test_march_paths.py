@@ -382,3 +382,63 @@ def test_phases_of_many_turns(name, n, kernel):
         got, fd = np.zeros(300), far.field_desc()
         L.check(sb.load().smp_field_values(C.byref(fd), 0.0, 300, C.c_void_p(pts.ctypes.data), C.c_void_p(got.ctypes.data)))
         assert np.array_equal(got, n_far)
+
+
+@pytest.mark.gpu
+def test_sweep_films_from_replayed_graphs(monkeypatch):
+    """A sweep of more photons than the pool has slots, its batches replayed from a graph (a fixed chunk: no
+    launch goes without), launched one by one, and as one launch: the films up to the order of their sums."""
+    setup = sb.config_plain_small(spatial_x=24, spatial_y=20, path_length_bins=4, er_stepsize=1.6e-4, **MIXED)
+    insts = [dict(mode=m, n_max=1e-3 + 3e-4 * m, n_clip=1e-3, f_u=0.7e6 + 2e5 * m, n_photons=400000, seed=60 + m) for m in range(3)]
+    monkeypatch.setenv("SMP_TUNE", "0")
+    out = []
+    for graph, direct in (("1", "0"), ("0", "0"), ("0", "10000000")):
+        monkeypatch.setenv("SMP_WF_CHUNK", "32")
+        monkeypatch.setenv("SMP_WF_GRAPH", graph)
+        monkeypatch.setenv("SMP_WF_DIRECT", direct)
+        films, st = sb.render_batch(setup, insts)
+        assert (st.launches == 1) == (direct != "0")
+        out.append((films, st.photons, st.er_steps, st.splats))
+    for films, *counts in out[1:]:
+        assert tuple(counts) == out[0][1:]
+        assert np.abs(films - out[0][0]).sum() <= 1e-12 * np.abs(films).sum()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("step", [1e-5, 2.9e-4, 3.4e-4])
+def test_spline_gradient_of_scattered_light_around_the_sweeps_chunk(step):
+    """Vertices, connections and reflections in segments of about 1000, 35 and 30 points and more, so that a
+    segment's turns and ends fall everywhere in the sweep's groups of 32: differences of matched paths along the
+    gradient itself, to the 3e-2 of the other fields' scattering tests. A photon's end granularity, 3e-8 m at the
+    long steps, is 1e-2 or so of its shift, random over the photons: 1e-3 of the sum."""
+    from test_adjoint import matched_fd
+    s = sb.config_spline(24, 4, max_depth=7, er_stepsize=step)
+    G = sb.roi_weights(s, 32)
+    n = 50_000
+    grad, st = sb.adjoint(s, n, G)
+    assert st.dropped == st.skipped == st.aborted == st.replay_mismatch == 0
+    th = sb.field_params(s)
+    d = grad * (3e-6 * np.sqrt(grad.size) / np.linalg.norm(grad))
+    up, dn = (th + d).astype(np.float32), (th - d).astype(np.float32)
+    predicted = float(grad @ (up.astype(np.float64) - dn.astype(np.float64)))
+    fd, frac = matched_fd(s, sb.with_field_params(s, up), sb.with_field_params(s, dn), n, G)
+    assert frac > 0.99
+    assert abs(predicted - fd) <= 3e-2 * abs(fd), (predicted, fd)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("setup", [lambda: sb.config_plain_small(mode=1, seed=70), lambda: sb.config_planewave(seed=71),
+                                   lambda: sb.config_spline(24, 4)], ids=["bessel", "wave", "spline"])
+def test_adjoint_traced_by_lanes(setup, monkeypatch):
+    """The checkpointing trace as one persistent launch (SMP_ADJ_TRACE=lanes) against the slot pool's: the same
+    photons, so the same gradient to the order of its double sums."""
+    s = dataclasses.replace(setup(), spatial_x=64, spatial_y=64, path_length_bins=8)
+    G, out = sb.roi_weights(s, 48), []
+    for lanes in (False, True):
+        if lanes:
+            monkeypatch.setenv("SMP_ADJ_TRACE", "lanes")
+        grad, st = sb.adjoint(s, 8000, G)
+        out.append((grad, st.photons, st.er_steps_forward, st.er_steps_replay, st.points, st.splats))
+        assert st.dropped == st.replay_mismatch == 0
+    assert out[0][1:] == out[1][1:]
+    assert np.abs(out[0][0] - out[1][0]).max() <= 1e-9 * np.abs(out[0][0]).max()
