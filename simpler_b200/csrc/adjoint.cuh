@@ -880,10 +880,11 @@ __device__ __forceinline__ void restore(Lane &L, const KParams &P, const AdjVert
 
 
 // Checkpointing trace: the render's persistent lane loop over the batch's photons with the
-// recording hook (no film is written: P.X = 0).
+// recording hook (no film is written: P.X = 0). Two blocks for the spline's 64 kept taps, as in the other
+// lane loops: with four they were spilled (20,000 photons on the 64^3 grid: 127 against 72 ms).
 template <int FK>
-__global__ void __launch_bounds__(128, 4) adjoint_trace_kernel(const __grid_constant__ KParams P,
-                                                               const __grid_constant__ AdjParams A) {
+__global__ void __launch_bounds__(128, lane_blocks(FK)) adjoint_trace_kernel(const __grid_constant__ KParams P,
+                                                                             const __grid_constant__ AdjParams A) {
     const int lane = threadIdx.x & 31;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     Lane L;
