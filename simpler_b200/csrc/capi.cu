@@ -667,14 +667,17 @@ static int plan_setup_field(smp_plan *p, const smp_field_desc &f) {
         SMP_CUDA(cudaMalloc(&p->d_coeff, delta.size() * sizeof(float)));
         SMP_CUDA(cudaMemcpy(p->d_coeff, delta.data(), delta.size() * sizeof(float), cudaMemcpyHostToDevice));
         p->kp.field.coeff = p->d_coeff;
-        std::vector<float4> quads;
-        spline_quads(f.grid_n, delta, quads);
         cudaFree(p->d_coeff4);
         p->d_coeff4 = nullptr;
-        SMP_CUDA(cudaMalloc(&p->d_coeff4, quads.size() * sizeof(float4)));
-        SMP_CUDA(cudaMemcpy(p->d_coeff4, quads.data(), quads.size() * sizeof(float4), cudaMemcpyHostToDevice));
-        p->kp.field.coeff4 = p->d_coeff4 + 1;              // entry x = 0 of the first row
-        p->kp.field.qrow = f.grid_n[0] + 2;
+        // the kernels index the quads in 32 bits; a grid whose padded rows pass them reads tap by tap
+        if (size_t(f.grid_n[0] + 2) * f.grid_n[1] * f.grid_n[2] <= 0x7fffffff) {
+            std::vector<float4> quads;
+            spline_quads(f.grid_n, delta, quads);
+            SMP_CUDA(cudaMalloc(&p->d_coeff4, quads.size() * sizeof(float4)));
+            SMP_CUDA(cudaMemcpy(p->d_coeff4, quads.data(), quads.size() * sizeof(float4), cudaMemcpyHostToDevice));
+            p->kp.field.coeff4 = p->d_coeff4 + 1;          // entry x = 0 of the first row
+            p->kp.field.qrow = f.grid_n[0] + 2;
+        }
         // bricks for the slot pool's march kernel (opts.spline_bricks): the padded quads and a tiled
         // TMA map over them
         const int nbx = (f.grid_n[0] + kSplineBrick - 1) / kSplineBrick, nby = (f.grid_n[1] + kSplineBrick - 1) / kSplineBrick,
