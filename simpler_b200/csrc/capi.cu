@@ -562,11 +562,18 @@ struct smp_plan {
     bool tuned = false;         // the schedule came from smp_plan_tune
     size_t wave_cap = 0;        // slots the pool allocation holds
     // Renders of at most two photons per lane of the tail kernel's grid (one for the spline) are one launch
-    // of that kernel, with no pool (SMP_WF_DIRECT: of at most that many photons; -1: this rule). Resident plans
-    // of Bessel and plane-wave fields take the same time either way up to 2.6 photons a lane (60,000 to
-    // 200,000 photons: 13.4 to 19.8 against 13.3 to 18.8 ms, mode 0), and a one-shot render is spared
-    // the pool's 150 MB and a hundred launches (120,000 photons 30 to 25 ms). The spline's pool pays
-    // sooner: 9,000 photons take 54 ms either way, 200,000 213 against 160.
+    // of that kernel, with no pool (SMP_WF_DIRECT: of at most that many photons; -1: this rule). Device ms of
+    // one launch / the pool on the plain small scene, and what spares a one-shot call the pool's 150 MB and a
+    // hundred launches on top (mode 0, 120,000 photons: 30 to 25 ms of the call):
+    //   mode 0         3,000 photons 8.0 / 13.1   60,000: 13.0 / 12.1   150,000: 15.0 / 15.0
+    //   mode 5         3,000: 29 / 37             60,000: 38 / 37       150,000: 43 to 45 / 41 to 44
+    //   two waves      3,000: 7.1 / 15.6          60,000: 15.0 / 14.9   150,000: 21.0 / 19.9
+    //   eight waves    3,000: 20.9 / 38.0         60,000: 37.8 / 37.3   150,000: 48.8 / 47.8
+    //   200 sources    20,000: 142 / 172          60,000: 172 / 194     150,000: 214 / 212
+    //   2,000 sources  20,000: 257 / 372          60,000: 277 / 389     150,000: 357 / 495
+    //   sweep of 12    32,000: 17.8 / 20.3        81,000: 25.0 / 23.4   129,000: 26.2 / 24.6
+    // A box with 40 % of its length in gaps, where no window reaches, loses (3,000: 16 / 21, 60,000: 29 / 24,
+    // 150,000: 31 / 27). The spline's pool pays sooner: 9,000 photons 48 / 54, 37,000 78 / 80, 200,000 213 / 160.
     long long direct_max = -1;
     long long pool_traces = 0;      // traces that took the pool since the last clear
     int wave_batch = 16;        // march/event launch pairs between live-slot checks

@@ -1108,7 +1108,7 @@ __global__ void __launch_bounds__(128, lane_blocks(FK)) march_kernel(const __gri
 // runs over the arcs' rows: a source's x depends on its row and (y, z) on its place in the row, so a
 // point's squared distance in (y, z) to each of the row's nt places is worked out once (in shared memory,
 // four to a 16-byte load, a column of its own per thread) and a term is one FMA, the reciprocal square
-// root, the phase and one cosine: 16 instructions instead of the 33 with the gradient, and two
+// root, the phase and one cosine: 15 instructions instead of the 33 with the gradient, and two
 // conversion-pipe operations instead of three, which bound it (16 cycles a term and scheduler).
 static constexpr int kValuesBlock = 128;
 static __global__ void __launch_bounds__(kValuesBlock)
