@@ -563,8 +563,8 @@ struct smp_plan {
     size_t wave_cap = 0;        // slots the pool allocation holds
     // Renders of at most two photons per lane of the tail kernel's grid (one for the spline) are one launch
     // of that kernel, with no pool (SMP_WF_DIRECT: of at most that many photons; -1: this rule). Device ms of
-    // one launch / the pool on the plain small scene, and what spares a one-shot call the pool's 150 MB and a
-    // hundred launches on top (mode 0, 120,000 photons: 30 to 25 ms of the call):
+    // one launch / the pool on the plain small scene; a one-shot call is spared the pool's 150 MB and a hundred
+    // launches besides (mode 0, 120,000 photons: the call 30 to 25 ms):
     //   mode 0         3,000 photons 8.0 / 13.1   60,000: 13.0 / 12.1   150,000: 15.0 / 15.0
     //   mode 5         3,000: 29 / 37             60,000: 38 / 37       150,000: 43 to 45 / 41 to 44
     //   two waves      3,000: 7.1 / 15.6          60,000: 15.0 / 14.9   150,000: 21.0 / 19.9
