@@ -330,7 +330,10 @@ def test_adjoint_of_a_brick_plan_marches_without_the_bricks_memory(tmp_path):
         plan.close()
     prof.export_chrome_trace(str(tmp_path / "trace.json"))
     events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
-    marches = [e["args"] for e in events if e.get("cat") == "kernel" and "wf_march_kernel" in e["name"]]
+    kernels = [e for e in events if e.get("cat") == "kernel"]
+    if not kernels:
+        pytest.skip("the profiler records no kernels on this machine")
+    marches = [e["args"] for e in kernels if "wf_march_kernel" in e["name"]]
     assert marches and all(m["shared memory"] < 16384 for m in marches), marches[:1]
 
 
