@@ -90,7 +90,8 @@ typedef struct smp_field_desc {
     double  center1[3], center2[3];
     /* plane waves (new field type): n = n_o + sum_i a_i sin(k_i . x - tau + phase_i),
        tau = phi_min + (phi_max - phi_min) * u is the per-photon temporal phase drawn where the
-       reference draws its Bessel 'scaling' (photon.cpp:324) */
+       reference draws its Bessel 'scaling' (photon.cpp:324). A phase_i, a phi_min or a source's phase of
+       more than ten turns is taken without its whole turns. */
     int32_t n_waves;
     int32_t _pad1;
     double  wave_amp[SMP_MAX_WAVES];
